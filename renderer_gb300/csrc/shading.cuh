@@ -44,9 +44,36 @@ __device__ __forceinline__ V3f normalize(V3f a) {
   float s = rsqrtf(l2);
   return {a.x * s, a.y * s, a.z * s};
 }
+__device__ __forceinline__ V3f reflect(V3f v, V3f n) { return v - (2.f * dot(v, n)) * n; }
+// a.y b.z - a.z b.y and so on, |a|^2 and a weighted sum of three vectors with
+// their fused multiply-adds spelled out. A sampled direction decides which
+// surface the path meets next, so it has to come out the same bit for bit in
+// every kernel; left to the compiler, which product of a sum is fused depends
+// on the code around it.
+__device__ __forceinline__ V3f cross_fused(V3f a, V3f b) {
+  return {__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)),
+          __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x))};
+}
+__device__ __forceinline__ float dot_fused(V3f a, V3f b) {
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ V3f normalize_fused(V3f a) {
+  const float l2 = dot_fused(a, a);
+  if (!(l2 > 1e-24f)) return {0.f, 0.f, 0.f};
+  const float s = rsqrtf(l2);
+  return {__fmul_rn(a.x, s), __fmul_rn(a.y, s), __fmul_rn(a.z, s)};
+}
+__device__ __forceinline__ V3f reflect_fused(V3f v, V3f n) {
+  const float s = -2.f * dot_fused(v, n);
+  return {__fmaf_rn(s, n.x, v.x), __fmaf_rn(s, n.y, v.y), __fmaf_rn(s, n.z, v.z)};
+}
+__device__ __forceinline__ V3f weighted_fused(V3f w, V3f a, V3f b, V3f c) {
+  return {__fmaf_rn(w.z, c.x, __fmaf_rn(w.y, b.x, __fmul_rn(w.x, a.x))),
+          __fmaf_rn(w.z, c.y, __fmaf_rn(w.y, b.y, __fmul_rn(w.x, a.y))),
+          __fmaf_rn(w.z, c.z, __fmaf_rn(w.y, b.z, __fmul_rn(w.x, a.z)))};
+}
 __device__ __forceinline__ bool is_zero(V3f a) { return a.x == 0.f && a.y == 0.f && a.z == 0.f; }
 __device__ __forceinline__ int signum(float x) { return (0.f < x) - (x < 0.f); }
-__device__ __forceinline__ V3f reflect(V3f v, V3f n) { return v - (2.f * dot(v, n)) * n; }
 __device__ __forceinline__ V3f ld3(const float* p) { return {p[0], p[1], p[2]}; }
 
 // ---------------------------------------------------------------- RNG -----
@@ -82,7 +109,7 @@ __device__ __forceinline__ unsigned dim_light(int D, int k) { return 3u + 2u * u
 // ----------------------------------------------------------- Sampling -----
 // Cosine-power direction about w, src/sampler.cpp:48-76 (opening angle pi/2).
 __device__ __forceinline__ V3f cosine_power_dir(V3f w, float sx, float sy, float e, float& pdf) {
-  w = normalize(w);
+  w = normalize_fused(w);
   float ie = 1.f / (e + 1.f);
   float z = powf(sx, ie);
   float r = sqrtf(fmaxf(0.f, 1.f - powf(sx, 2.f * ie)));
@@ -95,9 +122,9 @@ __device__ __forceinline__ V3f cosine_power_dir(V3f w, float sx, float sy, float
   if (ax < ay && ax < az) v = v3(0.f, w.z, -w.y);
   else if (ay < az) v = v3(w.z, 0.f, -w.x);
   else v = v3(w.y, -w.x, 0.f);
-  v = normalize(v);
-  V3f u = cross(v, w);
-  return normalize(nd.x * u + nd.y * v + nd.z * w);
+  v = normalize_fused(v);
+  V3f u = cross_fused(v, w);
+  return normalize_fused(weighted_fused(nd, u, v, w));
 }
 
 // ---------------------------------------------------------------- CSG -----
@@ -295,7 +322,7 @@ __device__ __forceinline__ V3f out_direction(const DeviceScene& S, const Vertex&
     }
     case kMatMirror:
       pdf = 1.f;
-      return reflect(h.d, h.n);
+      return reflect_fused(h.d, h.n);
     case kMatPhong: {
       V3f n = h.n;
       if (dot(h.d, n) > 0.f) n = -n;
