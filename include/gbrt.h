@@ -284,7 +284,9 @@ typedef struct gbrt_render_params {
 
 typedef enum gbrt_render_flags {
   /* Time every extend / shade / shadow kernel with CUDA events on the
-   * render stream (gbrt_stats *_ms fields). */
+   * render stream (gbrt_stats *_ms fields). Either flag makes the render
+   * launch these kernels for every bounce; without them small wavefronts and
+   * the last paths of large ones run whole in one launch. */
   GBRT_RENDER_TIME_KERNELS = 1,
   /* Count BVH nodes visited and primitives tested (gbrt_stats counters);
    * slower, for measurement only. */

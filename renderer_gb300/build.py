@@ -23,6 +23,13 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "-Xcompiler", "-fno-strict-aliasing", "-I", os.path.join(HERE, "..", "include")]
 
 
+# The path tracer's arithmetic has its fused multiply-adds spelled out: a path
+# comes out the same bit for bit in every kernel that runs it (one bounce per
+# launch, whole paths, many images). Left to the compiler, which product of a
+# sum is fused depends on the code around it.
+FLAGS = {"pathtrace.cu": ["-fmad=false"]}
+
+
 def nvcc():
     for cand in (os.environ.get("NVCC"), shutil.which("nvcc"), "/usr/local/cuda/bin/nvcc"):
         if cand and os.path.exists(cand):
@@ -41,7 +48,7 @@ def _compile(src, out=OUT, extra=()):
     obj = os.path.join(out, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
     lang = [] if src.endswith(".cu") else ["-x", "c++"]
-    cmd = [nvcc()] + ARCH + COMMON + list(extra) + lang + ["-c", path, "-o", obj]
+    cmd = [nvcc()] + ARCH + COMMON + FLAGS.get(src, []) + list(extra) + lang + ["-c", path, "-o", obj]
     if src.endswith(".cu"):
         cmd += ["-Xptxas", "-v"] if os.environ.get("GBRT_PTXAS_VERBOSE") else []
     r = subprocess.run(cmd, capture_output=True, text=True)

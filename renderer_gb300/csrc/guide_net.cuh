@@ -394,8 +394,8 @@ __device__ __forceinline__ float mixture_pdf(const float4* M, float x, float y, 
 #pragma unroll
   for (int k = 0; k < kLobes; ++k) {
     float4 l = M[2 + k];
-    float d = l.x * x + l.y * y + l.z * z;
-    q += cs[k] * __expf(l.w * (d - 1.f));
+    float d = __fmaf_rn(l.z, z, __fmaf_rn(l.x, x, __fmul_rn(l.y, y)));
+    q = __fmaf_rn(cs[k], __expf(l.w * (d - 1.f)), q);
   }
   return q;
 }
@@ -415,20 +415,21 @@ __device__ __forceinline__ void mixture_sample(const float4* M, float u0, float 
   float4 l = M[2 + k];
   float kap = l.w;
   // cos of the angle to the mean (inversion of the vMF marginal)
-  float w = 1.f + logf(u1 + (1.f - u1) * expf(-2.f * kap)) / kap;
+  float w = 1.f + logf(__fmaf_rn(1.f - u1, expf(-2.f * kap), u1)) / kap;
   w = fminf(fmaxf(w, -1.f), 1.f);
-  float sw = sqrtf(fmaxf(0.f, 1.f - w * w));
+  float sw = sqrtf(fmaxf(0.f, __fmaf_rn(-w, w, 1.f)));
   float sn, cs;
   sincospif(2.f * u2, &sn, &cs);
   // orthonormal basis about the mean (Duff et al. 2017)
   float sg = copysignf(1.f, l.z);
   float a = -1.f / (sg + l.z);
   float b = l.x * l.y * a;
-  float tx = 1.f + sg * l.x * l.x * a, ty = sg * b, tz = -sg * l.x;
-  float bx = b, by = sg + l.y * l.y * a, bz = -l.y;
-  x = sw * (cs * tx + sn * bx) + w * l.x;
-  y = sw * (cs * ty + sn * by) + w * l.y;
-  z = sw * (cs * tz + sn * bz) + w * l.z;
+  float tx = __fmaf_rn(sg * l.x * l.x, a, 1.f), ty = sg * b, tz = -sg * l.x;
+  float bx = b, by = __fmaf_rn(l.y * l.y, a, sg), bz = -l.y;
+  // (the multiply-adds spelled out, as in shading.cuh)
+  x = __fmaf_rn(sw, __fmaf_rn(sn, bx, __fmul_rn(cs, tx)), __fmul_rn(w, l.x));
+  y = __fmaf_rn(sw, __fmaf_rn(cs, ty, __fmul_rn(sn, by)), __fmul_rn(w, l.y));
+  z = __fmaf_rn(sw, __fmaf_rn(cs, tz, __fmul_rn(sn, bz)), __fmul_rn(w, l.z));
 }
 
 }  // namespace guide

@@ -113,7 +113,7 @@ struct PTState {
   float4* sh_ray;  // shadow queue: (o, tmin), (d, tmax)
   float4* sh_c;    // contribution, ignore prim in w (int bits)
   int* sh_slot;
-  int* counts;     // [0], [1] extension counts, [2] shadow count
+  int* counts;     // [0], [1] extension counts, [2] shadow count, [3] not 0: k_finish ran the last paths
   int ext_cap, sh_cap;  // entries of each extension queue and of the shadow queue (0: not checked)
   unsigned long long* work;   // work counters of the persistent kernels
   unsigned long long* tally;  // [0] extension rays, [1] shadow rays, [2] non-finite samples
@@ -217,13 +217,14 @@ __device__ __forceinline__ void start_path(const PTParams& P, const PTState& st,
 __device__ __forceinline__ void camera_dir(const PTParams& P, float sxp, float syp, float& dx, float& dy, float& dz) {
   float x = P.cam.l + (P.cam.r - P.cam.l) * (sxp + 0.5f) / float(P.cam.W);
   float y = P.cam.t + (P.cam.b - P.cam.t) * (syp + 0.5f) / float(P.cam.H);
-  dx = x * P.cam.u[0] + y * P.cam.v[0] - P.cam.w[0];
-  dy = x * P.cam.u[1] + y * P.cam.v[1] - P.cam.w[1];
-  dz = x * P.cam.u[2] + y * P.cam.v[2] - P.cam.w[2];
+  dx = mad2<0>(x, P.cam.u[0], y, P.cam.v[0]) - P.cam.w[0];
+  dy = mad2<0>(x, P.cam.u[1], y, P.cam.v[1]) - P.cam.w[1];
+  dz = mad2<0>(x, P.cam.u[2], y, P.cam.v[2]) - P.cam.w[2];
 }
 
-// The camera ray of the path in slot (path index P.g0 + slot of its image).
-__device__ __forceinline__ void raygen_slot(const PTParams& P, const PTState& st, int slot) {
+// The camera ray and the length of the path in slot (path index P.g0 + slot of
+// its image).
+__device__ __forceinline__ void camera_path(const PTParams& P, int slot, int& plen, float& dx, float& dy, float& dz) {
   unsigned long long g = P.g0 + (unsigned long long)slot;
   int pixel, s;
   if (P.idx32) {
@@ -239,10 +240,15 @@ __device__ __forceinline__ void raygen_slot(const PTParams& P, const PTState& st
   unsigned long long key = stream_key(P.seed, g);
   float sxp = float(px) + (stream_u(key, 0) + float(a)) / float(P.xs);
   float syp = float(py) + (stream_u(key, 1) + float(b)) / float(P.ys);
-  float dx, dy, dz;
   camera_dir(P, sxp, syp, dx, dy, dz);
   // The physical estimator plays Russian roulette per vertex instead.
-  const int plen = P.physical ? P.D : ref_path_length(P, stream_u(key, 2));
+  plen = P.physical ? P.D : ref_path_length(P, stream_u(key, 2));
+}
+
+__device__ __forceinline__ void raygen_slot(const PTParams& P, const PTState& st, int slot) {
+  int plen;
+  float dx, dy, dz;
+  camera_path(P, slot, plen, dx, dy, dz);
   start_path(P, st, slot, plen, dx, dy, dz);
 }
 
@@ -250,6 +256,7 @@ __global__ void __launch_bounds__(256) k_raygen(PTParams P, PTState st) {
   int slot = blockIdx.x * blockDim.x + threadIdx.x;
   if (slot == 0) {
     st.counts[0] = P.nb;
+    st.counts[3] = 0;
     st.work[0] = 0;  // work counter of the first extend
   }
   if (slot >= P.nb) return;
@@ -280,9 +287,10 @@ __device__ __forceinline__ void warp_add_counters(TraceCounters c, unsigned long
 // MS: the scene of each ray is its job's (gbrt_render_batch_fused).
 template <bool COUNT, bool WT, int STACK, bool GEN, bool MS>
 __device__ __forceinline__ void extend_body(const DeviceScene& S, const PTState& st, int cur, const BatchDev& bt) {
-  const int n = st.counts[cur];
+  const int n = st.counts[3] ? 0 : st.counts[cur];  // k_finish may have run the last paths
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st.tally[0] += (unsigned long long)n;
+    if (n == 0) st.counts[cur] = 0;
     st.counts[cur ^ 1] = 0;
     st.counts[2] = 0;
     st.work[cur ^ 1] = 0;
@@ -406,24 +414,54 @@ __device__ __forceinline__ void push_ext(const PTState& st, int nxt, int slot, V
   st.ext_slot[nxt][e] = slot;
 }
 
-__device__ __forceinline__ void load_pending(const PTState& st, int slot, Vertex& pv, V3f& pa, int& k) {
-  float4 pp = st.pv_p[slot], pn = st.pv_n[slot], pd = st.pv_d[slot], a = st.pv_a[slot];
-  pv.p = v3(pp.x, pp.y, pp.z);
-  pv.n = v3(pn.x, pn.y, pn.z);
-  pv.d = v3(pd.x, pd.y, pd.z);
-  pv.mat = __float_as_int(pp.w);
-  pv.tu = pd.w;
-  pv.tv = a.w;
-  pa = v3(a.x, a.y, a.z);
-  k = __float_as_int(pn.w);
-}
+// What the shading of a vertex reads and writes of its path. WaveState: the
+// arrays and queues of a wavefront; the rays it pushes are traced by the next
+// launches. PathState (k_path): registers of the thread that runs the path.
+struct WaveState {
+  const PTState& st;
+  int slot, nxt;  // path, extension queue to push to
+  __device__ __forceinline__ int4 ctl() const { return st.ctl[slot]; }
+  __device__ __forceinline__ void set_ctl(int i, int plen, int z, int w) { st.ctl[slot] = make_int4(i, plen, z, w); }
+  __device__ __forceinline__ float4 radiance() const { return st.L[slot]; }
+  __device__ __forceinline__ void set_radiance(float4 L) { st.L[slot] = L; }
+  __device__ __forceinline__ float4 alpha() const { return st.alpha[slot]; }
+  __device__ __forceinline__ void set_alpha(float4 a) { st.alpha[slot] = a; }
+  __device__ __forceinline__ void load_pending(Vertex& pv, V3f& pa, int& k) const {
+    float4 pp = st.pv_p[slot], pn = st.pv_n[slot], pd = st.pv_d[slot], a = st.pv_a[slot];
+    pv.p = v3(pp.x, pp.y, pp.z);
+    pv.n = v3(pn.x, pn.y, pn.z);
+    pv.d = v3(pd.x, pd.y, pd.z);
+    pv.mat = __float_as_int(pp.w);
+    pv.tu = pd.w;
+    pv.tv = a.w;
+    pa = v3(a.x, a.y, a.z);
+    k = __float_as_int(pn.w);
+  }
+  __device__ __forceinline__ void store_pending(const Vertex& v, V3f a, int k) {
+    st.pv_p[slot] = make_float4(v.p.x, v.p.y, v.p.z, __int_as_float(v.mat));
+    st.pv_n[slot] = make_float4(v.n.x, v.n.y, v.n.z, __int_as_float(k));
+    st.pv_d[slot] = make_float4(v.d.x, v.d.y, v.d.z, v.tu);
+    st.pv_a[slot] = make_float4(a.x, a.y, a.z, v.tv);
+  }
+  __device__ __forceinline__ void push(V3f p, V3f d) { push_ext(st, nxt, slot, p, d); }
+  // A shadow ray and what it adds to the radiance when nothing but primitive
+  // `ignore` is in its way.
+  __device__ __forceinline__ void shadow(V3f o, V3f d, float tmax, V3f c, int ignore) {
+    int e = agg_push(&st.counts[2]);
+    if (!in_range(st.sh_cap == 0 || e < st.sh_cap, st.err)) return;
+    st.sh_ray[2 * e] = make_float4(o.x, o.y, o.z, kEps);
+    st.sh_ray[2 * e + 1] = make_float4(d.x, d.y, d.z, tmax);
+    st.sh_c[e] = make_float4(c.x, c.y, c.z, __int_as_float(ignore));
+    st.sh_slot[e] = slot;
+  }
+};
 
 // Next-event estimation at a stored vertex: UniDiPathTracingIntegrator lines
 // 83-99 with Light::getIntensity for light lightIndex[k]. A non-zero
-// contribution goes to the shadow queue with its shadow ray.
-template <bool EXT, class R>
-__device__ __forceinline__ void nee(const DeviceScene& S, const PTParams& P, const PTState& st, int slot,
-                                    const R& rs, const Vertex& vx, V3f alpha, int k) {
+// contribution goes to the path's state with its shadow ray.
+template <bool EXT, class R, class ST>
+__device__ __forceinline__ void nee(const DeviceScene& S, const PTParams& P, ST& ss, const R& rs, const Vertex& vx,
+                                    V3f alpha, int k) {
   if (S.n_lights <= 0 || vx.mat < 0) return;
   unsigned dl = dim_light(P.D, k);
   float lx = rs.u(dl), ly = rs.u(dl + 1);
@@ -433,7 +471,7 @@ __device__ __forceinline__ void nee(const DeviceScene& S, const PTParams& P, con
   float stmax;
   int ignore = -1;
   if (Lt.type == GBRT_LIGHT_AREA) {
-    V3f lp = ld3(Lt.origin) + lx * ld3(Lt.u) + ly * ld3(Lt.v);
+    V3f lp = madv(ly, ld3(Lt.v), madv(lx, ld3(Lt.u), ld3(Lt.origin)));
     dir = vx.p - lp;
     Le = area_intensity(Lt, dir);
     sd = -normalize(dir);
@@ -468,12 +506,7 @@ __device__ __forceinline__ void nee(const DeviceScene& S, const PTParams& P, con
   float ac = fabsf(inCos);
   V3f c = v3(alpha.x * f.x * Le.x * ac, alpha.y * f.y * Le.y * ac, alpha.z * f.z * Le.z * ac);
   if (is_zero(c)) return;
-  int e = agg_push(&st.counts[2]);
-  if (!in_range(st.sh_cap == 0 || e < st.sh_cap, st.err)) return;
-  st.sh_ray[2 * e] = make_float4(vx.p.x, vx.p.y, vx.p.z, kEps);
-  st.sh_ray[2 * e + 1] = make_float4(sd.x, sd.y, sd.z, stmax);
-  st.sh_c[e] = make_float4(c.x, c.y, c.z, __int_as_float(ignore));
-  st.sh_slot[e] = slot;
+  ss.shadow(vx.p, sd, stmax, c, ignore);
 }
 
 // Shading of the hit at the head of one path: the body of the loop of
@@ -489,169 +522,168 @@ __device__ __forceinline__ void nee(const DeviceScene& S, const PTParams& P, con
 // Cornell box, 2^20 paths: 1.19 -> 1.06 ms a frame; ten small mesh scenes in
 // shared wavefronts 12.4 -> 11.0 ms; the 67M-path icosphere frame 51.5 ->
 // 49.8 ms (latency and the path state's traffic bound it there).
+template <bool EXT, class R, class ST>
+__device__ __forceinline__ void shade_vertex(const DeviceScene& S, const PTParams& P, ST& ss, const R& rs,
+                                             const RawHit& h, const int* hit_inst, float4 ro, float4 rd, int* err) {
+  if (!in_range(h.rec < S.n_recs && h.rec >= -1 - S.n_planes, err)) return;
+  int4 c = ss.ctl();
+  int i = c.x, plen = c.y, nst = c.z;
+  const bool pend = c.w != 0;
+  const V3f d = v3(rd.x, rd.y, rd.z);
+  const bool envHit = h.rec == -1 && S.env_light >= 0 && isinf(rd.w) && rd.w > 0.f;
+  Vertex vx;
+  vx.p = v3(0.f, 0.f, 0.f);
+  vx.n = vx.p;
+  vx.d = d;
+  vx.mat = -1;
+  vx.tu = 0.f;
+  vx.tv = 0.f;
+  V3f out = vx.p, alpha = vx.p;
+  int k = 0;
+  bool neePend = false, neeHere = false, store = false, push = false;
+  const bool missed = h.rec == -1 && !envHit;
+  int light = -1;
+  if (missed) {
+    // The path leaves the scene: the last stored vertex gets NEE (line 85).
+    neePend = pend;
+  } else if (envHit) {
+    light = S.env_light;
+    vx.p = normalize(d);  // point at infinity (w = 0)
+    vx.n = -vx.p;
+  } else {
+    vx.p = madv(h.t, d, v3(ro.x, ro.y, ro.z));
+    if (h.rec >= 0) {
+      const int4 m = __ldg(&S.meta[h.rec]);
+      const float4* rp = S.recs + 3 * int64_t(h.rec);
+      const float4 a = __ldg(rp);
+      const int kind = __float_as_int(a.w);
+      vx.mat = m.y;
+      light = m.w;
+      if (!in_range(light < S.n_lights && vx.mat < S.n_materials, err)) return;
+      if (EXT && S.tri_uv) hit_texcoords(S, h.rec, h.u, h.v, vx.p, vx.tu, vx.tv);
+      if (kind == kRecTriangle) {
+        if (m.z >= 0) {
+          const float* nn = S.tri_nrm + 12 * int64_t(m.z);
+          float w0 = 1.f - h.u - h.v;
+          vx.n = normalize(mad3v<0>(w0, ld3(nn), h.u, ld3(nn + 3), h.v, ld3(nn + 6)));
+        } else {
+          const float4 b = __ldg(rp + 1), cc = __ldg(rp + 2);
+          V3f p1 = v3(a.x, a.y, a.z), p2 = v3(b.x, b.y, b.z), p3 = v3(cc.x, cc.y, cc.z);
+          vx.n = normalize(cross(p1 - p2, p1 - p3));
+        }
+      } else if (kind == kRecSphere) {
+        vx.n = normf<0>(vx.p - v3(a.x, a.y, a.z));
+      } else if (EXT && kind == kRecCSG) {
+        csg_surface(S, __float_as_int(h.u), v3(ro.x, ro.y, ro.z), d, vx.p, vx.n, vx.mat, vx.tu, vx.tv);
+      } else {
+        vx.n = ld3(S.lights[light].nhat);
+      }
+      if (EXT && S.inst) {
+        const int in = *hit_inst;
+        if (in >= 0) vx.n = instance_normal(S, in, vx.n);
+      }
+    } else {
+      const float4 pl = __ldg(&S.planes[-2 - h.rec]);
+      vx.n = normalize(v3(pl.x, pl.y, pl.z));
+      vx.mat = S.plane_meta[-2 - h.rec].y;
+    }
+  }
+  if (light >= 0) {
+    // Emitter. Its own next-event term is zero (Material::brdf of a light
+    // is zero), so only its emission matters; the path ends here.
+    V3f e = envHit ? env_get(S, vx.p) : area_intensity(S.lights[light], -d);
+    float4 L4 = ss.radiance();
+    if (nst == 0) {
+      // The first stored vertex is an emitter: its emission is the sample.
+      L4.x = e.x; L4.y = e.y; L4.z = e.z;
+    } else if (pend) {
+      // The pending vertex sees this emitter (lines 70-81).
+      Vertex pv; V3f pa; int pk;
+      ss.load_pending(pv, pa, pk);
+      V3f dir = envHit ? -vx.p : pv.p - vx.p;
+      V3f f = brdf_eval<EXT>(S, pv, dir);
+      float inCos = dot(-normalize(dir), pv.n);
+      float outCos = dot(-normalize(pv.d), pv.n);
+      if (signum(inCos) == signum(outCos)) {
+        float ac = fabsf(inCos);
+        L4.x = __fmaf_rn(pa.x * f.x * e.x, ac, L4.x);
+        L4.y = __fmaf_rn(pa.y * f.y * e.y, ac, L4.y);
+        L4.z = __fmaf_rn(pa.z * f.z * e.z, ac, L4.z);
+      }
+    }
+    ss.set_radiance(L4);
+  } else if (!missed) {
+    float pdf;
+    V3f f;
+    out = out_direction<EXT>(S, vx, rs.u(dim_path(i)), rs.u(dim_path(i) + 1), pdf, f);
+    if (mat_specular(S.materials, vx.mat)) {
+      // Specular vertices are not stored (lines 87-91).
+      if (i == plen - 1 && plen < P.D) plen++;
+      i++;
+      push = i < plen;
+      neePend = !push && pend;
+    } else {
+      // Stored, non-specular vertex k = nst (lines 92-102): the previous
+      // pending vertex is now known not to be followed by an emitter.
+      neePend = pend;
+      const float4 a4 = ss.alpha();
+      alpha = v3(a4.x, a4.y, a4.z);
+      k = nst++;
+      bool ends = pdf == 0.f || is_zero(alpha);
+      V3f na = alpha;
+      if (!ends) {
+        float sc = fabsf(dotf<1>(normf<1>(out), vx.n)) / pdf;
+        na = v3(alpha.x * f.x * sc, alpha.y * f.y * sc, alpha.z * f.z * sc);
+        if (i > 3) {
+          float ir = 1.f / P.rr_pdf;
+          na = v3(na.x * ir, na.y * ir, na.z * ir);
+        }
+        i++;
+        ends = i >= plen;
+      }
+      // Without a next vertex this one is the last stored: its next-event
+      // estimation is due now too.
+      neeHere = ends;
+      store = push = !ends;
+      if (store) ss.set_alpha(make_float4(na.x, na.y, na.z, 0.f));
+    }
+  }
+  Vertex nv = vx;
+  V3f nalpha = alpha;
+  int nk = k;
+  if (neePend) ss.load_pending(nv, nalpha, nk);
+  if (store) ss.store_pending(vx, alpha, k);
+  if (push) {
+    ss.set_ctl(i, plen, nst, (store || (pend && !neePend)) ? 1 : 0);
+    ss.push(vx.p, out);
+  }
+  // A path that ends with a pending vertex before it owes two estimates.
+  bool both = neePend && neeHere;
+  bool due = neePend || neeHere;
+  while (due) {
+    nee<EXT>(S, P, ss, rs, nv, nalpha, nk);
+    due = both;
+    if (both) {
+      nv = vx;
+      nalpha = alpha;
+      nk = k;
+      both = false;
+    }
+  }
+}
+
 template <bool EXT, class R, bool MS>
 __device__ __forceinline__ void shade_body(const DeviceScene& S0, const PTParams& P0, const PTState& st, int cur,
                                            const BatchDev& bt) {
   const int n = st.counts[cur];
-  const int nxt = cur ^ 1;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int slot = st.ext_slot[cur][q];
     const int job = MS ? int(bt.job_of[slot]) : 0;
     const DeviceScene& S = MS ? bt.scenes[job] : S0;
     const PTParams& P = MS ? bt.jobs[job].P : P0;
-    const RawHit h = st.hits[q];
-    if (!in_range(h.rec < S.n_recs && h.rec >= -1 - S.n_planes, st.err)) continue;
-    const float4 ro = st.ext[cur][2 * q], rd = st.ext[cur][2 * q + 1];
-    int4 c = st.ctl[slot];
-    int i = c.x, plen = c.y, nst = c.z;
-    const bool pend = c.w != 0;
-    const R rs(P, slot);
-    const V3f d = v3(rd.x, rd.y, rd.z);
-    const bool envHit = h.rec == -1 && S.env_light >= 0 && isinf(rd.w) && rd.w > 0.f;
-    Vertex vx;
-    vx.p = v3(0.f, 0.f, 0.f);
-    vx.n = vx.p;
-    vx.d = d;
-    vx.mat = -1;
-    vx.tu = 0.f;
-    vx.tv = 0.f;
-    V3f out = vx.p, alpha = vx.p;
-    int k = 0;
-    bool neePend = false, neeHere = false, store = false, push = false;
-    const bool missed = h.rec == -1 && !envHit;
-    int light = -1;
-    if (missed) {
-      // The path leaves the scene: the last stored vertex gets NEE (line 85).
-      neePend = pend;
-    } else if (envHit) {
-      light = S.env_light;
-      vx.p = normalize(d);  // point at infinity (w = 0)
-      vx.n = -vx.p;
-    } else {
-      vx.p = v3(ro.x, ro.y, ro.z) + h.t * d;
-      if (h.rec >= 0) {
-        const int4 m = __ldg(&S.meta[h.rec]);
-        const float4* rp = S.recs + 3 * int64_t(h.rec);
-        const float4 a = __ldg(rp);
-        const int kind = __float_as_int(a.w);
-        vx.mat = m.y;
-        light = m.w;
-        if (!in_range(light < S.n_lights && vx.mat < S.n_materials, st.err)) continue;
-        if (EXT && S.tri_uv) hit_texcoords(S, h.rec, h.u, h.v, vx.p, vx.tu, vx.tv);
-        if (kind == kRecTriangle) {
-          if (m.z >= 0) {
-            const float* nn = S.tri_nrm + 12 * int64_t(m.z);
-            float w0 = 1.f - h.u - h.v;
-            vx.n = normalize(w0 * ld3(nn) + h.u * ld3(nn + 3) + h.v * ld3(nn + 6));
-          } else {
-            const float4 b = __ldg(rp + 1), cc = __ldg(rp + 2);
-            V3f p1 = v3(a.x, a.y, a.z), p2 = v3(b.x, b.y, b.z), p3 = v3(cc.x, cc.y, cc.z);
-            vx.n = normalize(cross(p1 - p2, p1 - p3));
-          }
-        } else if (kind == kRecSphere) {
-          vx.n = normalize(vx.p - v3(a.x, a.y, a.z));
-        } else if (EXT && kind == kRecCSG) {
-          csg_surface(S, __float_as_int(h.u), v3(ro.x, ro.y, ro.z), d, vx.p, vx.n, vx.mat, vx.tu, vx.tv);
-        } else {
-          vx.n = ld3(S.lights[light].nhat);
-        }
-        if (EXT && S.inst) {
-          const int in = st.hit_inst[q];
-          if (in >= 0) vx.n = instance_normal(S, in, vx.n);
-        }
-      } else {
-        const float4 pl = __ldg(&S.planes[-2 - h.rec]);
-        vx.n = normalize(v3(pl.x, pl.y, pl.z));
-        vx.mat = S.plane_meta[-2 - h.rec].y;
-      }
-    }
-    if (light >= 0) {
-      // Emitter. Its own next-event term is zero (Material::brdf of a light
-      // is zero), so only its emission matters; the path ends here.
-      V3f e = envHit ? env_get(S, vx.p) : area_intensity(S.lights[light], -d);
-      float4 L4 = st.L[slot];
-      if (nst == 0) {
-        // The first stored vertex is an emitter: its emission is the sample.
-        L4.x = e.x; L4.y = e.y; L4.z = e.z;
-      } else if (pend) {
-        // The pending vertex sees this emitter (lines 70-81).
-        Vertex pv; V3f pa; int pk;
-        load_pending(st, slot, pv, pa, pk);
-        V3f dir = envHit ? -vx.p : pv.p - vx.p;
-        V3f f = brdf_eval<EXT>(S, pv, dir);
-        float inCos = dot(-normalize(dir), pv.n);
-        float outCos = dot(-normalize(pv.d), pv.n);
-        if (signum(inCos) == signum(outCos)) {
-          float ac = fabsf(inCos);
-          L4.x += pa.x * f.x * e.x * ac;
-          L4.y += pa.y * f.y * e.y * ac;
-          L4.z += pa.z * f.z * e.z * ac;
-        }
-      }
-      st.L[slot] = L4;
-    } else if (!missed) {
-      float pdf;
-      V3f f;
-      out = out_direction<EXT>(S, vx, rs.u(dim_path(i)), rs.u(dim_path(i) + 1), pdf, f);
-      if (mat_specular(S.materials, vx.mat)) {
-        // Specular vertices are not stored (lines 87-91).
-        if (i == plen - 1 && plen < P.D) plen++;
-        i++;
-        push = i < plen;
-        neePend = !push && pend;
-      } else {
-        // Stored, non-specular vertex k = nst (lines 92-102): the previous
-        // pending vertex is now known not to be followed by an emitter.
-        neePend = pend;
-        const float4 a4 = st.alpha[slot];
-        alpha = v3(a4.x, a4.y, a4.z);
-        k = nst++;
-        bool ends = pdf == 0.f || is_zero(alpha);
-        V3f na = alpha;
-        if (!ends) {
-          float sc = fabsf(dot(normalize(out), vx.n)) / pdf;
-          na = v3(alpha.x * f.x * sc, alpha.y * f.y * sc, alpha.z * f.z * sc);
-          if (i > 3) {
-            float ir = 1.f / P.rr_pdf;
-            na = v3(na.x * ir, na.y * ir, na.z * ir);
-          }
-          i++;
-          ends = i >= plen;
-        }
-        // Without a next vertex this one is the last stored: its next-event
-        // estimation is due now too.
-        neeHere = ends;
-        store = push = !ends;
-        if (store) st.alpha[slot] = make_float4(na.x, na.y, na.z, 0.f);
-      }
-    }
-    Vertex nv = vx;
-    V3f nalpha = alpha;
-    int nk = k;
-    if (neePend) load_pending(st, slot, nv, nalpha, nk);
-    if (store) {
-      st.pv_p[slot] = make_float4(vx.p.x, vx.p.y, vx.p.z, __int_as_float(vx.mat));
-      st.pv_n[slot] = make_float4(vx.n.x, vx.n.y, vx.n.z, __int_as_float(k));
-      st.pv_d[slot] = make_float4(d.x, d.y, d.z, vx.tu);
-      st.pv_a[slot] = make_float4(alpha.x, alpha.y, alpha.z, vx.tv);
-    }
-    if (push) {
-      st.ctl[slot] = make_int4(i, plen, nst, (store || (pend && !neePend)) ? 1 : 0);
-      push_ext(st, nxt, slot, vx.p, out);
-    }
-    // A path that ends with a pending vertex before it owes two estimates.
-    bool both = neePend && neeHere;
-    bool due = neePend || neeHere;
-    while (due) {
-      nee<EXT>(S, P, st, slot, rs, nv, nalpha, nk);
-      due = both;
-      if (both) {
-        nv = vx;
-        nalpha = alpha;
-        nk = k;
-        both = false;
-      }
-    }
+    WaveState ss{st, slot, cur ^ 1};
+    shade_vertex<EXT>(S, P, ss, R(P, slot), st.hits[q], EXT ? st.hit_inst + q : nullptr, st.ext[cur][2 * q],
+                      st.ext[cur][2 * q + 1], st.err);
   }
 }
 
@@ -678,9 +710,10 @@ __global__ void __launch_bounds__(256, 4) k_shade_ms(PTState st, int cur, BatchD
 // otherwise (one-sample MIS: the pdf of either choice is the mixture
 // guide_frac q + (1 - guide_frac) p_bsdf, used in the throughput and in both
 // power heuristics).
-__device__ __forceinline__ void nee_phys(const DeviceScene& S, const PTState& st, int slot, unsigned long long key,
-                                         unsigned base, const PhysBsdf& b, V3f x, V3f n, V3f wo, V3f alpha,
-                                         const float4* M, float frac) {
+template <class ST>
+__device__ __forceinline__ void nee_phys(const DeviceScene& S, ST& ss, unsigned long long key, unsigned base,
+                                         const PhysBsdf& b, V3f x, V3f n, V3f wo, V3f alpha, const float4* M,
+                                         float frac) {
   const int nL = S.n_lights;
   const float pChoose = 1.f / float(nL);
   const int li = min(stream_index(key, base + 3, nL), nL - 1);
@@ -691,7 +724,7 @@ __device__ __forceinline__ void nee_phys(const DeviceScene& S, const PTState& st
   bool delta = false;
   int ignore = -1;
   if (Lt.type == GBRT_LIGHT_AREA) {
-    V3f y = ld3(Lt.origin) + lx * ld3(Lt.u) + ly * ld3(Lt.v);
+    V3f y = madv(ly, ld3(Lt.v), madv(lx, ld3(Lt.u), ld3(Lt.origin)));
     V3f d = y - x;
     dist = len(d);
     wi = normalize(d);
@@ -728,17 +761,12 @@ __device__ __forceinline__ void nee_phys(const DeviceScene& S, const PTState& st
   float pb;
   V3f f = phys_eval(b, n, wo, wi, pb);
   if (is_zero(f)) return;
-  if (M) pb = frac * guide::mixture_pdf(M, wi.x, wi.y, wi.z) + (1.f - frac) * pb;
+  if (M) pb = mad2<0>(frac, guide::mixture_pdf(M, wi.x, wi.y, wi.z), 1.f - frac, pb);
   float w = delta ? 1.f : power_heuristic(pl, pb);
   float sc = fabsf(dot(n, wi)) * w / pl;
   V3f c = v3(alpha.x * f.x * Le.x * sc, alpha.y * f.y * Le.y * sc, alpha.z * f.z * Le.z * sc);
   if (is_zero(c)) return;
-  int e = agg_push(&st.counts[2]);
-  if (!in_range(st.sh_cap == 0 || e < st.sh_cap, st.err)) return;
-  st.sh_ray[2 * e] = make_float4(x.x, x.y, x.z, kEps);
-  st.sh_ray[2 * e + 1] = make_float4(wi.x, wi.y, wi.z, isinf(dist) ? CUDART_INF_F : dist - kEps);
-  st.sh_c[e] = make_float4(c.x, c.y, c.z, __int_as_float(ignore));
-  st.sh_slot[e] = slot;
+  ss.shadow(x, wi, isinf(dist) ? CUDART_INF_F : dist - kEps, c, ignore);
 }
 
 // Normal (unflipped), material and texture coordinates of a surface hit that
@@ -758,7 +786,7 @@ __device__ __forceinline__ void surface_normal(const DeviceScene& S, const RawHi
       if (m.z >= 0) {
         const float* nn = S.tri_nrm + 12 * int64_t(m.z);
         float w0 = 1.f - h.u - h.v;
-        nrm = normalize(w0 * ld3(nn) + h.u * ld3(nn + 3) + h.v * ld3(nn + 6));
+        nrm = normalize(mad3v<0>(w0, ld3(nn), h.u, ld3(nn + 3), h.v, ld3(nn + 6)));
       } else {
         const float4 b = __ldg(rp + 1), cc = __ldg(rp + 2);
         V3f p1 = v3(a.x, a.y, a.z), p2 = v3(b.x, b.y, b.z), p3 = v3(cc.x, cc.y, cc.z);
@@ -768,7 +796,7 @@ __device__ __forceinline__ void surface_normal(const DeviceScene& S, const RawHi
       csg_surface(S, __float_as_int(h.u), o, d, x, nrm, mat, tu, tv);
       return;
     } else {
-      nrm = normalize(x - v3(a.x, a.y, a.z));  // sphere
+      nrm = normf<0>(x - v3(a.x, a.y, a.z));  // sphere
     }
     if (EXT && inst >= 0) nrm = instance_normal(S, inst, nrm);
     if (EXT && S.tri_uv) hit_texcoords(S, h.rec, h.u, h.v, x, tu, tv);
@@ -779,126 +807,134 @@ __device__ __forceinline__ void surface_normal(const DeviceScene& S, const RawHi
   }
 }
 
+// q: the vertex's place in the extension queue (its mixture, its records).
+template <bool GUIDED, bool EXT, class ST>
+__device__ __forceinline__ void shade_phys_vertex(const DeviceScene& S, const PTParams& P, ST& ss, int slot,
+                                                  const RawHit& h, const int* hit_inst, float4 ro, float4 rd,
+                                                  const PTState& st, int q) {
+  const float pChoose = S.n_lights > 0 ? 1.f / float(S.n_lights) : 0.f;
+  if (!in_range(h.rec < S.n_recs && h.rec >= -1 - S.n_planes, st.err)) return;
+  int4 c = ss.ctl();
+  const int i = c.x;
+  if (GUIDED && P.record && (c.z & kRecOpen)) {
+    // The radiance the path had gathered before this vertex: the rest of
+    // the path is what the last recorded direction brought in.
+    st.rec[size_t(kRecComp * ((c.z & 15) - 1) + 4) * st.nslots + slot] = st.L[slot];
+    c.z &= ~kRecOpen;
+  }
+  const bool prevSpec = c.w != 0;
+  const float4 a4 = ss.alpha();
+  const V3f alpha = v3(a4.x, a4.y, a4.z);
+  const float prevPdf = a4.w;
+  const V3f d = v3(rd.x, rd.y, rd.z);
+  const bool envHit = h.rec == -1 && S.env_light >= 0 && isinf(rd.w) && rd.w > 0.f;
+  if (h.rec == -1 && !envHit) return;
+  if (envHit) {
+    V3f dn = normalize(d);
+    V3f Le = env_get(S, dn);
+    float w = prevSpec ? 1.f : power_heuristic(prevPdf, pChoose * (S.env_marg ? env_pdf(S, dn) : 0.25f * kInvPi));
+    float4 L4 = ss.radiance();
+    L4.x = __fmaf_rn(alpha.x * Le.x, w, L4.x);
+    L4.y = __fmaf_rn(alpha.y * Le.y, w, L4.y);
+    L4.z = __fmaf_rn(alpha.z * Le.z, w, L4.z);
+    ss.set_radiance(L4);
+    return;
+  }
+  const V3f x = madv(h.t, d, v3(ro.x, ro.y, ro.z));
+  if (h.rec >= 0) {
+    const int lt = __ldg(&S.meta[h.rec]).w;
+    if (!in_range(lt < S.n_lights, st.err)) return;
+    if (lt >= 0) {
+      // An area light: emission on its front side (AreaLight is one-sided).
+      const DevLight& Lt = S.lights[lt];
+      float dl = len(d);
+      float cl = dot(-(1.f / dl) * d, ld3(Lt.nhat));
+      if (cl > 0.f) {
+        float w = 1.f;
+        if (!prevSpec) {
+          float dist = h.t * dl;
+          w = power_heuristic(prevPdf, pChoose * dist * dist / (cl * Lt.normal_len));
+        }
+        float4 L4 = ss.radiance();
+        L4.x = __fmaf_rn(alpha.x * Lt.intensity[0], w, L4.x);
+        L4.y = __fmaf_rn(alpha.y * Lt.intensity[1], w, L4.y);
+        L4.z = __fmaf_rn(alpha.z * Lt.intensity[2], w, L4.z);
+        ss.set_radiance(L4);
+      }
+      return;
+    }
+  }
+  V3f nrm;
+  int mat = -1;
+  float tu, tv;
+  surface_normal<EXT>(S, h, (EXT && S.inst) ? *hit_inst : -1, v3(ro.x, ro.y, ro.z), d, x, nrm, mat, tu, tv);
+  const PhysBsdf b = phys_bsdf<EXT>(S, mat, tu, tv);
+  if (b.kind <= 0) return;
+  const unsigned long long key = stream_key(P.seed, P.g0 + (unsigned long long)slot);
+  const unsigned base = dim_phys(i);
+  const V3f wo = -normalize(d);
+  const bool flipped = dot(nrm, wo) < 0.f;
+  if (flipped) nrm = -nrm;
+  const bool depthOk = P.guide_depth == 0 || i < P.guide_depth;
+  const bool guideHere = GUIDED && P.guided && depthOk && b.kind >= 1 && b.kind <= 3;
+  const float4* M = guideHere ? st.mix + guide::kMixStride * size_t(q) : nullptr;
+  if (b.kind <= 3 && S.n_lights > 0) nee_phys(S, ss, key, base, b, x, nrm, wo, alpha, M, P.guide_frac);
+  V3f wi, wgt;
+  float pdf;
+  bool spec;
+  const float u0 = stream_u(key, base), u1 = stream_u(key, base + 1), u2 = stream_u(key, base + 2);
+  if (guideHere) {
+    if (stream_u(key, base + 7) < P.guide_frac) {
+      guide::mixture_sample(M, u0, u1, u2, wi.x, wi.y, wi.z);
+    } else if (!phys_sample(b, nrm, wo, flipped, u0, u1, u2, wi, wgt, pdf, spec)) {
+      return;
+    }
+    float pb;
+    V3f f = phys_eval(b, nrm, wo, wi, pb);
+    pdf = mad2<0>(P.guide_frac, guide::mixture_pdf(M, wi.x, wi.y, wi.z), 1.f - P.guide_frac, pb);
+    if (is_zero(f) || !(pdf > 0.f)) return;
+    wgt = (dot(nrm, wi) / pdf) * f;
+    spec = false;
+  } else if (!phys_sample(b, nrm, wo, flipped, u0, u1, u2, wi, wgt, pdf, spec)) {
+    return;
+  }
+  V3f na = mulc(alpha, wgt);
+  if (i + 1 >= 3 && P.term_p > 0.f) {
+    if (stream_u(key, base + 6) < P.term_p) return;
+    na = (1.f / (1.f - P.term_p)) * na;
+  }
+  if (i + 1 >= P.D) return;
+  int z = 0;
+  if (GUIDED) {
+    z = c.z;
+    if (P.record && depthOk && b.kind >= 1 && b.kind <= 3 && (z & 15) < kRecords) {
+      const size_t r = size_t(kRecComp * (z & 15)) * st.nslots + slot;
+      const size_t ns = size_t(st.nslots);
+      st.rec[r] = make_float4(x.x, x.y, x.z, pdf);
+      st.rec[r + ns] = make_float4(nrm.x, nrm.y, nrm.z, wi.x);
+      st.rec[r + 2 * ns] = make_float4(wo.x, wo.y, wo.z, wi.y);
+      st.rec[r + 3 * ns] = make_float4(na.x, na.y, na.z, wi.z);
+      st.rec[r + 5 * ns] = make_float4((alpha.x + alpha.y + alpha.z) * (1.f / 3.f), alpha.x, alpha.y, alpha.z);
+      z = ((z & 15) + 1) | kRecOpen;
+    }
+  }
+  ss.set_alpha(make_float4(na.x, na.y, na.z, pdf));
+  ss.set_ctl(i + 1, c.y, z, spec ? 1 : 0);
+  ss.push(x, wi);
+}
+
 template <bool GUIDED, bool EXT, bool MS>
 __device__ __forceinline__ void shade_phys_body(const DeviceScene& S0, const PTParams& P0, const PTState& st,
                                                 int cur, const BatchDev& bt) {
   const int n = st.counts[cur];
-  const int nxt = cur ^ 1;
-  const float pChoose0 = MS ? 0.f : (S0.n_lights > 0 ? 1.f / float(S0.n_lights) : 0.f);
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int slot = st.ext_slot[cur][q];
     const int job = MS ? int(bt.job_of[slot]) : 0;
     const DeviceScene& S = MS ? bt.scenes[job] : S0;
     const PTParams& P = MS ? bt.jobs[job].P : P0;
-    const float pChoose = MS ? (S.n_lights > 0 ? 1.f / float(S.n_lights) : 0.f) : pChoose0;
-    const RawHit h = st.hits[q];
-    if (!in_range(h.rec < S.n_recs && h.rec >= -1 - S.n_planes, st.err)) continue;
-    const float4 ro = st.ext[cur][2 * q], rd = st.ext[cur][2 * q + 1];
-    int4 c = st.ctl[slot];
-    const int i = c.x;
-    if (GUIDED && P.record && (c.z & kRecOpen)) {
-      // The radiance the path had gathered before this vertex: the rest of
-      // the path is what the last recorded direction brought in.
-      st.rec[size_t(kRecComp * ((c.z & 15) - 1) + 4) * st.nslots + slot] = st.L[slot];
-      c.z &= ~kRecOpen;
-    }
-    const bool prevSpec = c.w != 0;
-    const float4 a4 = st.alpha[slot];
-    const V3f alpha = v3(a4.x, a4.y, a4.z);
-    const float prevPdf = a4.w;
-    const V3f d = v3(rd.x, rd.y, rd.z);
-    const bool envHit = h.rec == -1 && S.env_light >= 0 && isinf(rd.w) && rd.w > 0.f;
-    if (h.rec == -1 && !envHit) continue;
-    if (envHit) {
-      V3f dn = normalize(d);
-      V3f Le = env_get(S, dn);
-      float w = prevSpec ? 1.f : power_heuristic(prevPdf, pChoose * (S.env_marg ? env_pdf(S, dn) : 0.25f * kInvPi));
-      float4 L4 = st.L[slot];
-      L4.x += alpha.x * Le.x * w; L4.y += alpha.y * Le.y * w; L4.z += alpha.z * Le.z * w;
-      st.L[slot] = L4;
-      continue;
-    }
-    const V3f x = v3(ro.x, ro.y, ro.z) + h.t * d;
-    if (h.rec >= 0) {
-      const int lt = __ldg(&S.meta[h.rec]).w;
-      if (!in_range(lt < S.n_lights, st.err)) continue;
-      if (lt >= 0) {
-        // An area light: emission on its front side (AreaLight is one-sided).
-        const DevLight& Lt = S.lights[lt];
-        float dl = len(d);
-        float cl = dot(-(1.f / dl) * d, ld3(Lt.nhat));
-        if (cl > 0.f) {
-          float w = 1.f;
-          if (!prevSpec) {
-            float dist = h.t * dl;
-            w = power_heuristic(prevPdf, pChoose * dist * dist / (cl * Lt.normal_len));
-          }
-          float4 L4 = st.L[slot];
-          L4.x += alpha.x * Lt.intensity[0] * w;
-          L4.y += alpha.y * Lt.intensity[1] * w;
-          L4.z += alpha.z * Lt.intensity[2] * w;
-          st.L[slot] = L4;
-        }
-        continue;
-      }
-    }
-    V3f nrm;
-    int mat = -1;
-    float tu, tv;
-    surface_normal<EXT>(S, h, (EXT && S.inst) ? st.hit_inst[q] : -1, v3(ro.x, ro.y, ro.z), d, x, nrm, mat, tu, tv);
-    const PhysBsdf b = phys_bsdf<EXT>(S, mat, tu, tv);
-    if (b.kind <= 0) continue;
-    const unsigned long long key = stream_key(P.seed, P.g0 + (unsigned long long)slot);
-    const unsigned base = dim_phys(i);
-    const V3f wo = -normalize(d);
-    const bool flipped = dot(nrm, wo) < 0.f;
-    if (flipped) nrm = -nrm;
-    const bool depthOk = P.guide_depth == 0 || i < P.guide_depth;
-    const bool guideHere = GUIDED && P.guided && depthOk && b.kind >= 1 && b.kind <= 3;
-    const float4* M = guideHere ? st.mix + guide::kMixStride * size_t(q) : nullptr;
-    if (b.kind <= 3 && S.n_lights > 0) nee_phys(S, st, slot, key, base, b, x, nrm, wo, alpha, M, P.guide_frac);
-    V3f wi, wgt;
-    float pdf;
-    bool spec;
-    const float u0 = stream_u(key, base), u1 = stream_u(key, base + 1), u2 = stream_u(key, base + 2);
-    if (guideHere) {
-      if (stream_u(key, base + 7) < P.guide_frac) {
-        guide::mixture_sample(M, u0, u1, u2, wi.x, wi.y, wi.z);
-      } else if (!phys_sample(b, nrm, wo, flipped, u0, u1, u2, wi, wgt, pdf, spec)) {
-        continue;
-      }
-      float pb;
-      V3f f = phys_eval(b, nrm, wo, wi, pb);
-      pdf = P.guide_frac * guide::mixture_pdf(M, wi.x, wi.y, wi.z) + (1.f - P.guide_frac) * pb;
-      if (is_zero(f) || !(pdf > 0.f)) continue;
-      wgt = (dot(nrm, wi) / pdf) * f;
-      spec = false;
-    } else if (!phys_sample(b, nrm, wo, flipped, u0, u1, u2, wi, wgt, pdf, spec)) {
-      continue;
-    }
-    V3f na = mulc(alpha, wgt);
-    if (i + 1 >= 3 && P.term_p > 0.f) {
-      if (stream_u(key, base + 6) < P.term_p) continue;
-      na = (1.f / (1.f - P.term_p)) * na;
-    }
-    if (i + 1 >= P.D) continue;
-    int z = 0;
-    if (GUIDED) {
-      z = c.z;
-      if (P.record && depthOk && b.kind >= 1 && b.kind <= 3 && (z & 15) < kRecords) {
-        const size_t r = size_t(kRecComp * (z & 15)) * st.nslots + slot;
-        const size_t ns = size_t(st.nslots);
-        st.rec[r] = make_float4(x.x, x.y, x.z, pdf);
-        st.rec[r + ns] = make_float4(nrm.x, nrm.y, nrm.z, wi.x);
-        st.rec[r + 2 * ns] = make_float4(wo.x, wo.y, wo.z, wi.y);
-        st.rec[r + 3 * ns] = make_float4(na.x, na.y, na.z, wi.z);
-        st.rec[r + 5 * ns] = make_float4((alpha.x + alpha.y + alpha.z) * (1.f / 3.f), alpha.x, alpha.y, alpha.z);
-        z = ((z & 15) + 1) | kRecOpen;
-      }
-    }
-    st.alpha[slot] = make_float4(na.x, na.y, na.z, pdf);
-    st.ctl[slot] = make_int4(i + 1, c.y, z, spec ? 1 : 0);
-    push_ext(st, nxt, slot, x, wi);
+    WaveState ss{st, slot, cur ^ 1};
+    shade_phys_vertex<GUIDED, EXT>(S, P, ss, slot, st.hits[q], EXT ? st.hit_inst + q : nullptr, st.ext[cur][2 * q],
+                                   st.ext[cur][2 * q + 1], st, q);
   }
 }
 
@@ -910,6 +946,122 @@ __global__ void __launch_bounds__(256, 4) k_shade_phys(DeviceScene S, PTParams P
 template <bool EXT>
 __global__ void __launch_bounds__(256, 4) k_shade_phys_ms(PTState st, int cur, BatchDev bt) {
   shade_phys_body<false, EXT, true>(bt.scenes[0], bt.jobs[0].P, st, cur, bt);
+}
+
+// ---------------------------------------------------------- whole paths ----
+// The state of a path that one thread runs from its camera ray to its end.
+// Nothing of it goes through memory; shadow rays are traced on the spot.
+template <int STACK, bool GEN>
+struct PathState {
+  const DeviceScene& S;
+  int* err;
+  int4 c;
+  float4 L, a;
+  Vertex pv;
+  V3f pa;
+  int pk;
+  V3f no, nd;   // the next ray
+  bool go;      // the path goes on along it
+  unsigned shadows;
+  __device__ __forceinline__ int4 ctl() const { return c; }
+  __device__ __forceinline__ void set_ctl(int i, int plen, int z, int w) { c = make_int4(i, plen, z, w); }
+  __device__ __forceinline__ float4 radiance() const { return L; }
+  __device__ __forceinline__ void set_radiance(float4 v) { L = v; }
+  __device__ __forceinline__ float4 alpha() const { return a; }
+  __device__ __forceinline__ void set_alpha(float4 v) { a = v; }
+  __device__ __forceinline__ void load_pending(Vertex& v, V3f& va, int& k) const { v = pv; va = pa; k = pk; }
+  __device__ __forceinline__ void store_pending(const Vertex& v, V3f va, int k) { pv = v; pa = va; pk = k; }
+  __device__ __forceinline__ void push(V3f p, V3f d) { no = p; nd = d; go = true; }
+  __device__ __forceinline__ void shadow(V3f o, V3f d, float tmax, V3f cc, int ignore) {
+    ++shadows;
+    const TRay r = make_tray(make_float4(o.x, o.y, o.z, kEps), make_float4(d.x, d.y, d.z, tmax));
+    float t, u, v;
+    if (trace_ray<true, false, false, STACK, GEN>(S, r, ignore, t, u, v, err, nullptr) == -1) {
+      L.x += cc.x;
+      L.y += cc.y;
+      L.z += cc.z;
+    }
+  }
+};
+
+// Runs the path whose next ray is (ro, rd) to its end; rays traced so far in
+// ext.
+template <bool PHYS, bool EXT, class R, int STACK, bool GEN>
+__device__ __forceinline__ void run_path(const DeviceScene& S, const PTParams& P, const PTState& st, int slot,
+                                         const R& rs, PathState<STACK, GEN>& ss, float4 ro, float4 rd, unsigned& ext) {
+  for (int it = 0; it < P.D; ++it) {
+    RawHit h;
+    int32_t inst = -1;
+    h.rec = trace_ray<false, false, false, STACK, GEN>(S, make_tray(ro, rd), -1, h.t, h.u, h.v, st.err, nullptr, &inst);
+    ++ext;
+    ss.go = false;
+    if (PHYS) shade_phys_vertex<false, EXT>(S, P, ss, slot, h, &inst, ro, rd, st, 0);
+    else shade_vertex<EXT>(S, P, ss, rs, h, &inst, ro, rd, st.err);
+    if (!ss.go) break;
+    ro = make_float4(ss.no.x, ss.no.y, ss.no.z, kEps);
+    rd = make_float4(ss.nd.x, ss.nd.y, ss.nd.z, CUDART_INF_F);
+  }
+}
+
+__device__ __forceinline__ void tally_rays(const PTState& st, unsigned ext, unsigned shadows) {
+  for (int o = 16; o > 0; o >>= 1) {
+    ext += __shfl_xor_sync(0xffffffffu, ext, o);
+    shadows += __shfl_xor_sync(0xffffffffu, shadows, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (ext) atomicAdd(&st.tally[0], (unsigned long long)ext);
+    if (shadows) atomicAdd(&st.tally[1], (unsigned long long)shadows);
+  }
+}
+
+// A small wavefront in one launch instead of 3 D + 1: every thread runs one
+// path from the camera ray to its end and writes its radiance.
+template <bool PHYS, bool EXT, bool GEN, int STACK>
+__global__ void __launch_bounds__(kTraceBlock, 4) k_path(DeviceScene S, PTParams P, PTState st) {
+  unsigned ext = 0, shadows = 0;
+  const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot < P.nb) {
+    PathState<STACK, GEN> ss{S, st.err};
+    int plen;
+    float dx, dy, dz;
+    camera_path(P, slot, plen, dx, dy, dz);
+    ss.c = make_int4(0, plen, 0, PHYS ? 1 : 0);
+    ss.L = make_float4(0.f, 0.f, 0.f, 0.f);
+    ss.a = make_float4(1.f, 1.f, 1.f, 0.f);
+    ss.shadows = 0;
+    run_path<PHYS, EXT>(S, P, st, slot, StreamSrc(P, slot), ss,
+                        make_float4(P.cam.eye[0], P.cam.eye[1], P.cam.eye[2], kEps),
+                        make_float4(dx, dy, dz, CUDART_INF_F), ext);
+    st.L[slot] = ss.L;
+    shadows = ss.shadows;
+  }
+  tally_rays(st, ext, shadows);
+}
+
+// The last paths of a wavefront in one launch: when at most `limit` rays wait
+// in the extension queue cur, every thread takes one and runs its path to the
+// end; counts[3] then tells the launches of the remaining bounces that
+// nothing is left. With more rays it does nothing.
+template <bool PHYS, bool EXT, bool GEN, class R, int STACK>
+__global__ void __launch_bounds__(kTraceBlock, 4) k_finish(DeviceScene S, PTParams P, PTState st, int cur, int limit) {
+  const int n = st.counts[cur];
+  if (n > limit || n == 0) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) st.counts[3] = 1;
+  unsigned ext = 0, shadows = 0;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int slot = st.ext_slot[cur][q];
+    PathState<STACK, GEN> ss{S, st.err};
+    ss.c = st.ctl[slot];
+    ss.L = st.L[slot];
+    ss.a = st.alpha[slot];
+    ss.shadows = 0;
+    if (!PHYS && ss.c.w != 0) WaveState{st, slot, 0}.load_pending(ss.pv, ss.pa, ss.pk);
+    run_path<PHYS, EXT>(S, P, st, slot, R(P, slot), ss, st.ext[cur][2 * q], st.ext[cur][2 * q + 1], ext);
+    st.L[slot] = ss.L;
+    shadows += ss.shadows;
+  }
+  __syncwarp();
+  tally_rays(st, ext, shadows);
 }
 
 // ------------------------------------------------------------ guiding ----
@@ -925,7 +1077,7 @@ __global__ void __launch_bounds__(256) k_guide_prep(DeviceScene S, PTState st, i
     if (h.rec != -1 && !(h.rec >= 0 && __ldg(&S.meta[h.rec]).w >= 0)) {
       const float4 ro = st.ext[cur][2 * q], rd = st.ext[cur][2 * q + 1];
       const V3f d = v3(rd.x, rd.y, rd.z);
-      const V3f x = v3(ro.x, ro.y, ro.z) + h.t * d;
+      const V3f x = madv(h.t, d, v3(ro.x, ro.y, ro.z));
       V3f nrm;
       int mat = -1;
       float tu, tv;
@@ -1153,6 +1305,7 @@ __global__ void __launch_bounds__(1024) k_batch_begin(BatchDev bt, PTState st) {
   if (threadIdx.x == 0) {
     bt.cursor[1] = nb;
     st.counts[0] = int(nb);
+    st.counts[3] = 0;
     st.work[0] = 0;  // work counter of the first extend
   }
 }
@@ -1309,6 +1462,58 @@ static void (*pick_shade(const gbrt_scene* s, bool physical, bool guided))(Devic
   return ext ? k_shade_phys<false, true> : k_shade_phys<false, false>;
 }
 
+// The whole-path kernels of a render, null when it has none: watertight
+// triangles, trees deeper than the short stack and the injected small stack
+// take the kernels per bounce.
+struct PathKernels {
+  void (*path)(DeviceScene, PTParams, PTState) = nullptr;
+  void (*finish)(DeviceScene, PTParams, PTState, int, int) = nullptr;
+};
+template <bool PHYS, class R>
+static PathKernels path_kernels(const gbrt_scene* s) {
+  if (s->view.csg_prog || s->view.inst)
+    return {k_path<PHYS, true, true, kShortStack>, k_finish<PHYS, true, true, R, kShortStack>};
+  if (ext_scene(s)) return {k_path<PHYS, true, false, kShortStack>, k_finish<PHYS, true, false, R, kShortStack>};
+  return {k_path<PHYS, false, false, kShortStack>, k_finish<PHYS, false, false, R, kShortStack>};
+}
+static PathKernels pick_path(const gbrt_scene* s, bool physical) {
+  if (s->watertight || s->ctx->fault_small_stack || stack_need(s->max_depth4) > kShortStack) return {};
+  return physical ? path_kernels<true, StreamSrc>(s) : path_kernels<false, StreamSrc>(s);
+}
+
+// Threads of k_path / k_finish resident at once (launch bounds 128 x 4).
+static long long path_lanes(const gbrt_ctx* ctx) { return 512ll * ctx->num_sms; }
+
+// Wavefronts of up to this many paths take k_path. What it saves, the
+// latency of 3 D nearly empty launches, grows with the tree's depth; what it
+// costs, lanes that idle while their warp's longest path goes on, grows with
+// the paths per lane. Measured (frame time by bounces / by k_path, us): Cornell
+// box (one level) 131k paths 425 / 342, 262k 540 / 588; two rooms of 500,000
+// triangles 262k 1330 / 888, 524k 1729 / 1623; icosphere of 1.31M 262k
+// 2036 / 816, 1M 3132 / 2454.
+static long long whole_path_limit(const gbrt_scene* s) {
+  return path_lanes(s->ctx) * (8 + std::min(s->max_depth4, 16)) / 4;
+}
+
+// A small wavefront: blocks of one warp while that spreads it over more SMs.
+static void launch_path(const PathKernels& pk, const gbrt_scene* s, const PTParams& P, const PTState& st,
+                        cudaStream_t stream) {
+  const int block = P.nb <= s->ctx->num_sms * kTraceBlock ? 32 : kTraceBlock;
+  pk.path<<<(P.nb + block - 1) / block, block, 0, stream>>>(s->view, P, st);
+}
+
+// Ends the wavefront here when its extension queue holds at most one ray per
+// resident thread (4.2M paths, by bounces alone / with this before every
+// bounce from the third on: icosphere 8.24 / 7.68 ms, terrain 6.80 / 6.08,
+// two rooms 9.01 / 8.76; twice and four times that limit are slower on the
+// rooms and the Cornell box).
+static void launch_finish(const PathKernels& pk, const gbrt_scene* s, const PTParams& P, const PTState& st, int cur,
+                          cudaStream_t stream) {
+  const int limit = int(std::min<long long>(path_lanes(s->ctx), P.nb));
+  pk.finish<<<(limit + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, stream>>>(s->view, P, st, cur, limit);
+}
+constexpr int kFinishFrom = 2;  // first bounce that k_finish is launched before
+
 static void init_params(PTParams& P, const gbrt_ctx* ctx, const gbrt_camera& cam, const gbrt_render_params& prm,
                         unsigned long long total) {
   P.cam = make_camera(cam);
@@ -1379,36 +1584,51 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
   cudaError_t e = cudaSuccess;
   double* d_sum = d_sum_in;
   auto A = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-  A(buf.alloc(&st.alpha, B)); A(buf.alloc(&st.L, B)); A(buf.alloc(&st.ctl, B));
-  A(buf.alloc(&st.pv_p, B)); A(buf.alloc(&st.pv_n, B)); A(buf.alloc(&st.pv_d, B)); A(buf.alloc(&st.pv_a, B));
-  A(buf.alloc(&st.ext[0], 2 * B)); A(buf.alloc(&st.ext[1], 2 * B));
-  A(buf.alloc(&st.ext_slot[0], B)); A(buf.alloc(&st.ext_slot[1], B));
-  A(buf.alloc(&st.hits, B));
-  if (s->view.inst) A(buf.alloc(&st.hit_inst, B));
-  A(buf.alloc(&st.sh_ray, 4 * B)); A(buf.alloc(&st.sh_c, 2 * B)); A(buf.alloc(&st.sh_slot, 2 * B));
-  A(buf.alloc(&st.counts, 4)); A(buf.alloc(&st.work, 4)); A(buf.alloc(&st.tally, 8)); A(buf.alloc(&st.err, 1));
-  st.ext_cap = int(B);
-  st.sh_cap = int(2 * B);
+  const bool count = (prm->flags & GBRT_RENDER_COUNT_TRAVERSAL) != 0;
+  const bool timeK = (prm->flags & GBRT_RENDER_TIME_KERNELS) != 0;
+  // Per-kernel times and counters want the kernels per bounce.
+  const PathKernels pk = timeK || count ? PathKernels{} : pick_path(s, P.physical != 0);
+  // Every wavefront by k_path: of a path only its radiance is stored (the
+  // preview of 3,015 paths: 24 allocations cost 30 us of its 139).
+  const bool whole = pk.path && B <= whole_path_limit(s);
+  A(buf.alloc(&st.L, B));
+  A(buf.alloc(&st.alpha, whole ? 1 : B)); A(buf.alloc(&st.ctl, whole ? 1 : B));
+  A(buf.alloc(&st.counts, 4)); A(buf.alloc(&st.work, 4));
+  if (!whole) {
+    A(buf.alloc(&st.pv_p, B)); A(buf.alloc(&st.pv_n, B)); A(buf.alloc(&st.pv_d, B)); A(buf.alloc(&st.pv_a, B));
+    A(buf.alloc(&st.ext[0], 2 * B)); A(buf.alloc(&st.ext[1], 2 * B));
+    A(buf.alloc(&st.ext_slot[0], B)); A(buf.alloc(&st.ext_slot[1], B));
+    A(buf.alloc(&st.hits, B));
+    if (s->view.inst) A(buf.alloc(&st.hit_inst, B));
+    A(buf.alloc(&st.sh_ray, 4 * B)); A(buf.alloc(&st.sh_c, 2 * B)); A(buf.alloc(&st.sh_slot, 2 * B));
+    st.ext_cap = int(B);
+    st.sh_cap = int(2 * B);
+  }
+  // The tallies and the error word, cleared and read back together.
+  struct Tail {
+    unsigned long long tally[8];
+    int err, pad;
+  } *d_tail = nullptr, tail{};
+  A(buf.alloc(&d_tail, 1));
+  st.tally = reinterpret_cast<unsigned long long*>(d_tail);
+  st.err = reinterpret_cast<int*>(st.tally + 8);
   if (!d_sum) A(buf.alloc(&d_sum, npix * 3));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render buffers");
   if (!keep_sums) {
     A(cudaMemsetAsync(d_sum, 0, npix * 3 * sizeof(double), stream));
     if (d_sumsq) A(cudaMemsetAsync(d_sumsq, 0, npix * 3 * sizeof(double), stream));
   }
-  A(cudaMemsetAsync(st.tally, 0, 8 * sizeof(unsigned long long), stream));
-  A(cudaMemsetAsync(st.err, 0, sizeof(int), stream));
+  A(cudaMemsetAsync(d_tail, 0, sizeof(Tail), stream));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render set-up");
 
-  const bool count = (prm->flags & GBRT_RENDER_COUNT_TRAVERSAL) != 0;
-  const bool timeK = (prm->flags & GBRT_RENDER_TIME_KERNELS) != 0;
   const TraceKernels tk = pick_kernels(s, count);
   auto kExt = tk.ext;
   auto kSh = tk.sh;
   // Persistent grids: every SM filled with as many blocks as fit.
   int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kExt, kTraceBlock, 0);
+  if (!whole) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kExt, kTraceBlock, 0);
   const int traceGrid = std::max(1, per) * ctx->num_sms;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kSh, kTraceBlock, 0);
+  if (!whole) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kSh, kTraceBlock, 0);
   const int shadowGrid = std::max(1, per) * ctx->num_sms;
   const int shadeGrid = ctx->num_sms * 8;
   auto kShade = pick_shade(s, P.physical != 0, false);
@@ -1430,18 +1650,27 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
     if (stop && *stop) { status = fail(ctx, GBRT_ERR_CANCELLED, "gbrt_render: cancelled"); break; }
     P.g0 = g0;
     P.nb = int(std::min<unsigned long long>((unsigned long long)B, total - g0));
-    k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
-    ++launches;
-    for (int it = 0; it < P.D; ++it) {
-      int cur = it & 1;
-      if (timeK) mark();
-      kExt<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
-      if (timeK) mark();
-      kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
-      if (timeK) mark();
-      kSh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
-      if (timeK) mark();
-      launches += 3;
+    if (whole) {
+      launch_path(pk, s, P, st, stream);
+      ++launches;
+    } else {
+      k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
+      ++launches;
+      for (int it = 0; it < P.D; ++it) {
+        int cur = it & 1;
+        if (pk.finish && it >= kFinishFrom) {
+          launch_finish(pk, s, P, st, cur, stream);
+          ++launches;
+        }
+        if (timeK) mark();
+        kExt<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+        if (timeK) mark();
+        kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
+        if (timeK) mark();
+        kSh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
+        if (timeK) mark();
+        launches += 3;
+      }
     }
     launch_accumulate(P, st, d_sum, d_sumsq, stream);
     ++launches;
@@ -1454,11 +1683,10 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
   ++launches;
   cudaEventRecord(ev1, stream);
   A(cudaGetLastError());
-  unsigned long long tally[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int err = 0;
-  A(cudaMemcpyAsync(tally, st.tally, sizeof tally, cudaMemcpyDeviceToHost, stream));
-  A(cudaMemcpyAsync(&err, st.err, sizeof err, cudaMemcpyDeviceToHost, stream));
+  A(cudaMemcpyAsync(&tail, d_tail, sizeof tail, cudaMemcpyDeviceToHost, stream));
   A(cudaStreamSynchronize(stream));
+  const unsigned long long* tally = tail.tally;
+  const int err = tail.err;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ev0, ev1);
   cudaEventDestroy(ev0);
@@ -1627,19 +1855,26 @@ static gbrt_status render_noalloc_impl(gbrt_scene* s, const gbrt_camera* cam, co
   const int shadowGrid = std::max(1, per) * ctx->num_sms;
   const int shadeGrid = ctx->num_sms * 8;
   auto kShade = pick_shade(s, P.physical != 0, false);
+  const PathKernels pk =
+      (prm->flags & GBRT_RENDER_COUNT_TRAVERSAL) ? PathKernels{} : pick_path(s, P.physical != 0);
   auto t0 = std::chrono::steady_clock::now();
   unsigned long long launches = 0;
   for (unsigned long long g0 = 0; g0 < total; g0 += (unsigned long long)B) {
     P.g0 = g0;
     P.nb = int(std::min<unsigned long long>((unsigned long long)B, total - g0));
-    k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
-    ++launches;
-    for (int it = 0; it < P.D; ++it) {
-      int cur = it & 1;
-      kExt<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
-      kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
-      kSh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
-      launches += 3;
+    if (pk.path && P.nb <= whole_path_limit(s)) {
+      launch_path(pk, s, P, st, stream);
+      ++launches;
+    } else {
+      k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
+      ++launches;
+      for (int it = 0; it < P.D; ++it) {
+        int cur = it & 1;
+        kExt<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+        kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
+        kSh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
+        launches += 3;
+      }
     }
     launch_accumulate(P, st, d_sum, d_sumsq, stream);
     ++launches;
@@ -1952,31 +2187,38 @@ static gbrt_status render_guided_impl(gbrt_scene* s, const gbrt_camera* cam, con
     A(cudaMemsetAsync(d_pass, 0, n3 * sizeof(double), stream));
     if (record) A(cudaMemsetAsync(st.tcount, 0, sizeof(int), stream));
     auto kShade = pick_shade(s, true, P.guided || P.record);
+    // Passes that neither sample the guide nor record for it.
+    const PathKernels pk = P.guided || P.record ? PathKernels{} : pick_path(s, true);
     for (unsigned long long g0 = 0; g0 < passTotal && e == cudaSuccess; g0 += (unsigned long long)B) {
       P.g0 = g0;
       P.nb = int(std::min<unsigned long long>((unsigned long long)B, passTotal - g0));
-      k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
-      for (int it = 0; it < P.D; ++it) {
-        int cur = it & 1;
-        tk.ext<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
-        if (P.guided && (P.guide_depth == 0 || it < P.guide_depth)) {
-          cudaEvent_t ea = nullptr, eb = nullptr;
-          if (timeK) {
-            cudaEventCreate(&ea);
-            cudaEventCreate(&eb);
-            cudaEventRecord(ea, stream);
+      if (pk.path && P.nb <= whole_path_limit(s)) {
+        launch_path(pk, s, P, st, stream);
+      } else {
+        k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
+        for (int it = 0; it < P.D; ++it) {
+          int cur = it & 1;
+          if (pk.finish && it >= kFinishFrom) launch_finish(pk, s, P, st, cur, stream);
+          tk.ext<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+          if (P.guided && (P.guide_depth == 0 || it < P.guide_depth)) {
+            cudaEvent_t ea = nullptr, eb = nullptr;
+            if (timeK) {
+              cudaEventCreate(&ea);
+              cudaEventCreate(&eb);
+              cudaEventRecord(ea, stream);
+            }
+            k_guide_prep<<<shadeGrid, 256, 0, stream>>>(s->view, st, cur);
+            A(guide::launch_infer(g, st.gin, st.counts + cur, 0, st.mix, stream));
+            if (timeK) {
+              cudaEventRecord(eb, stream);
+              iev.push_back(ea);
+              iev.push_back(eb);
+            }
+            ++infer_launches;
           }
-          k_guide_prep<<<shadeGrid, 256, 0, stream>>>(s->view, st, cur);
-          A(guide::launch_infer(g, st.gin, st.counts + cur, 0, st.mix, stream));
-          if (timeK) {
-            cudaEventRecord(eb, stream);
-            iev.push_back(ea);
-            iev.push_back(eb);
-          }
-          ++infer_launches;
+          kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
+          tk.sh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
         }
-        kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
-        tk.sh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
       }
       launch_accumulate(P, st, d_pass, nullptr, stream);
       if (record) k_guide_collect<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);

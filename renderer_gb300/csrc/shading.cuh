@@ -31,50 +31,56 @@ __device__ __forceinline__ V3f operator-(V3f a, V3f b) { return {a.x - b.x, a.y 
 __device__ __forceinline__ V3f operator-(V3f a) { return {-a.x, -a.y, -a.z}; }
 __device__ __forceinline__ V3f operator*(float s, V3f a) { return {s * a.x, s * a.y, s * a.z}; }
 __device__ __forceinline__ V3f mulc(V3f a, V3f b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
-__device__ __forceinline__ float dot(V3f a, V3f b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ V3f cross(V3f a, V3f b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
-__device__ __forceinline__ float len2(V3f a) { return dot(a, a); }
-__device__ __forceinline__ float len(V3f a) { return sqrtf(dot(a, a)); }
-// QVector3D::normalized: the zero vector stays zero.
-__device__ __forceinline__ V3f normalize(V3f a) {
-  float l2 = dot(a, a);
-  if (!(l2 > 1e-24f)) return {0.f, 0.f, 0.f};
-  float s = rsqrtf(l2);
-  return {a.x * s, a.y * s, a.z * s};
-}
-__device__ __forceinline__ V3f reflect(V3f v, V3f n) { return v - (2.f * dot(v, n)) * n; }
-// a.y b.z - a.z b.y and so on, |a|^2 and a weighted sum of three vectors with
-// their fused multiply-adds spelled out. A sampled direction decides which
-// surface the path meets next, so it has to come out the same bit for bit in
-// every kernel; left to the compiler, which product of a sum is fused depends
+// This file's arithmetic is compiled without contraction (build.py FLAGS); the
+// fused multiply-adds are spelled out here, so that a path comes out the same
+// bit for bit in every kernel that runs it. A sampled direction decides which
+// surface the path meets next, and an exponent of 500 or a mirror makes a last
+// bit visible. Left to the compiler, which product of a sum it fuses depends
 // on the code around it.
-__device__ __forceinline__ V3f cross_fused(V3f a, V3f b) {
-  return {__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)),
-          __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x))};
+//
+// a b + c d with the first (F = 0) or the second product fused.
+template <int F>
+__device__ __forceinline__ float mad2(float a, float b, float c, float d) {
+  return F == 0 ? __fmaf_rn(a, b, __fmul_rn(c, d)) : __fmaf_rn(c, d, __fmul_rn(a, b));
 }
-__device__ __forceinline__ float dot_fused(V3f a, V3f b) {
-  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+template <int F>
+__device__ __forceinline__ float dotf(V3f a, V3f b) {
+  return __fmaf_rn(a.z, b.z, mad2<F>(a.x, b.x, a.y, b.y));
 }
-__device__ __forceinline__ float dot_fused_yx(V3f a, V3f b) {
-  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+// The same with the last product rounded: what refraction and the Blinn lobe
+// have always computed.
+__device__ __forceinline__ float dot_split(V3f a, V3f b) {
+  return mad2<1>(a.x, b.x, a.y, b.y) + a.z * b.z;
 }
-__device__ __forceinline__ V3f normalize_fused(V3f a) {
-  const float l2 = dot_fused(a, a);
+template <int F>
+__device__ __forceinline__ V3f normf(V3f a) {
+  const float l2 = dotf<F>(a, a);
   if (!(l2 > 1e-24f)) return {0.f, 0.f, 0.f};
   const float s = rsqrtf(l2);
   return {__fmul_rn(a.x, s), __fmul_rn(a.y, s), __fmul_rn(a.z, s)};
 }
-__device__ __forceinline__ V3f reflect_fused(V3f v, V3f n) {
-  const float s = -2.f * dot_fused(v, n);
-  return {__fmaf_rn(s, n.x, v.x), __fmaf_rn(s, n.y, v.y), __fmaf_rn(s, n.z, v.z)};
+template <int F>
+__device__ __forceinline__ V3f crossf3(V3f a, V3f b) {
+  return {mad2<F>(a.y, b.z, -a.z, b.y), mad2<F>(a.z, b.x, -a.x, b.z), mad2<F>(a.x, b.y, -a.y, b.x)};
 }
-__device__ __forceinline__ V3f weighted_fused(V3f w, V3f a, V3f b, V3f c) {
-  return {__fmaf_rn(w.z, c.x, __fmaf_rn(w.y, b.x, __fmul_rn(w.x, a.x))),
-          __fmaf_rn(w.z, c.y, __fmaf_rn(w.y, b.y, __fmul_rn(w.x, a.y))),
-          __fmaf_rn(w.z, c.z, __fmaf_rn(w.y, b.z, __fmul_rn(w.x, a.z)))};
+__device__ __forceinline__ V3f madv(float s, V3f a, V3f b) {
+  return {__fmaf_rn(s, a.x, b.x), __fmaf_rn(s, a.y, b.y), __fmaf_rn(s, a.z, b.z)};
 }
+template <int F>
+__device__ __forceinline__ V3f mad2v(float s, V3f a, float t, V3f b) {
+  return {mad2<F>(s, a.x, t, b.x), mad2<F>(s, a.y, t, b.y), mad2<F>(s, a.z, t, b.z)};
+}
+template <int F>
+__device__ __forceinline__ V3f mad3v(float s, V3f a, float t, V3f b, float u, V3f c) { return madv(u, c, mad2v<F>(s, a, t, b)); }
+template <int F>
+__device__ __forceinline__ V3f reflf(V3f v, V3f n) { return madv(-2.f * dotf<F>(v, n), n, v); }
+__device__ __forceinline__ float dot(V3f a, V3f b) { return dotf<0>(a, b); }
+__device__ __forceinline__ V3f cross(V3f a, V3f b) { return crossf3<0>(a, b); }
+__device__ __forceinline__ float len2(V3f a) { return dot(a, a); }
+__device__ __forceinline__ float len(V3f a) { return sqrtf(dot(a, a)); }
+// QVector3D::normalized: the zero vector stays zero.
+__device__ __forceinline__ V3f normalize(V3f a) { return normf<0>(a); }
+__device__ __forceinline__ V3f reflect(V3f v, V3f n) { return reflf<0>(v, n); }
 __device__ __forceinline__ bool is_zero(V3f a) { return a.x == 0.f && a.y == 0.f && a.z == 0.f; }
 __device__ __forceinline__ int signum(float x) { return (0.f < x) - (x < 0.f); }
 __device__ __forceinline__ V3f ld3(const float* p) { return {p[0], p[1], p[2]}; }
@@ -118,7 +124,7 @@ static __device__ __noinline__ float pow_shared(float x, float y) { return powf(
 // Cosine-power direction about w, src/sampler.cpp:48-76 (opening angle pi/2).
 // With exponent 1 two of the three powers are the number itself.
 __device__ __forceinline__ V3f cosine_power_dir(V3f w, float sx, float sy, float e, float& pdf) {
-  w = normalize_fused(w);
+  w = normf<0>(w);
   float ie = 1.f / (e + 1.f);
   float z = pow_shared(sx, ie);
   float r = sqrtf(fmaxf(0.f, 1.f - (e == 1.f ? sx : pow_shared(sx, 2.f * ie))));
@@ -131,9 +137,9 @@ __device__ __forceinline__ V3f cosine_power_dir(V3f w, float sx, float sy, float
   if (ax < ay && ax < az) v = v3(0.f, w.z, -w.y);
   else if (ay < az) v = v3(w.z, 0.f, -w.x);
   else v = v3(w.y, -w.x, 0.f);
-  v = normalize_fused(v);
-  V3f u = cross_fused(v, w);
-  return normalize_fused(weighted_fused(nd, u, v, w));
+  v = normf<0>(v);
+  V3f u = crossf3<0>(v, w);
+  return normf<0>(mad3v<1>(nd.x, u, nd.y, v, nd.z, w));
 }
 
 // ---------------------------------------------------------------- CSG -----
@@ -229,8 +235,7 @@ __device__ __forceinline__ void hit_texcoords(const DeviceScene& S, int rec, flo
 __device__ __forceinline__ V3f instance_normal(const DeviceScene& S, int in, V3f n) {
   const float4* M = S.inst + 4 * int64_t(in);
   const float4 m0 = __ldg(M), m1 = __ldg(M + 1), m2 = __ldg(M + 2);
-  return normalize(v3(m0.x * n.x + m1.x * n.y + m2.x * n.z, m0.y * n.x + m1.y * n.y + m2.y * n.z,
-                      m0.z * n.x + m1.z * n.y + m2.z * n.z));
+  return normalize(mad3v<0>(n.x, v3(m0.x, m0.y, m0.z), n.y, v3(m1.x, m1.y, m1.z), n.z, v3(m2.x, m2.y, m2.z)));
 }
 
 // TextureMaterial::get + brdf's pow (src/texturematerial.cpp:62-74): the
@@ -287,7 +292,7 @@ __device__ __forceinline__ V3f brdf_eval(const DeviceScene& S, const Vertex& h, 
       return v3(0.f, 0.f, 0.f);
     case kMatPhong: {
       V3f s = phong_spec(m, h, dir);
-      return v3(m.kd[0] * kInvPi + s.x, m.kd[1] * kInvPi + s.y, m.kd[2] * kInvPi + s.z);
+      return madv(kInvPi, ld3(m.kd), s);
     }
     case kMatBlinn: {
       V3f n = h.n;
@@ -298,7 +303,7 @@ __device__ __forceinline__ V3f brdf_eval(const DeviceScene& S, const Vertex& h, 
       V3f wh = normalize(wi + wo);
       float D = (m.exponent + 2.f) * (0.5f * kInvPi) * pow_shared(dot(wh, n), m.exponent);
       float f = D * blinn_G(wi, wo, n) / (4.f * dot(wo, n) * dot(wi, n));
-      return v3(m.kd[0] * kInvPi + m.ks[0] * f, m.kd[1] * kInvPi + m.ks[1] * f, m.kd[2] * kInvPi + m.ks[2] * f);
+      return mad2v<0>(kInvPi, ld3(m.kd), f, ld3(m.ks));
     }
     default:
       return v3(0.f, 0.f, 0.f);
@@ -309,6 +314,20 @@ __device__ __forceinline__ bool mat_specular(const DevMaterial* mats, int mat) {
   if (mat < 0) return false;
   int t = mats[mat].type;
   return t == kMatMirror || t == kMatTransparent;
+}
+
+// Fresnel reflection or refraction of the unit direction d at the side n of a
+// dielectric, chosen by u.
+__device__ __forceinline__ V3f refract_or_reflect(V3f d, V3f n, float ratio, float u) {
+  const float cosI = dot_split(-n, d);
+  const float s2 = fmaxf(0.f, __fmaf_rn(-cosI, cosI, 1.f));
+  const float sinO = ratio * sqrtf(s2);
+  const float cosO = sqrtf(fmaxf(0.f, __fmaf_rn(-(ratio * ratio), s2, 1.f)));
+  const float rPerp = __fmaf_rn(-ratio, cosO, cosI) / __fmaf_rn(ratio, cosO, cosI);
+  const float rPara = __fmaf_rn(ratio, cosI, -cosO) / __fmaf_rn(ratio, cosI, cosO);
+  const float R = 0.5f * mad2<0>(rPerp, rPerp, rPara, rPara);
+  if (sinO > 1.f || u < R) return madv(2.f * cosI, n, d);
+  return mad2v<0>(ratio, d, ratio * cosI - float(signum(cosI)) * cosO, n);
 }
 
 // Material::outDirection(hit, sample, pdf, brdf). The lobes only choose the
@@ -336,7 +355,7 @@ __device__ __forceinline__ V3f out_direction(const DeviceScene& S, const Vertex&
       break;
     case kMatMirror:
       pdf = 1.f;
-      return reflect_fused(h.d, h.n);
+      return reflf<0>(h.d, h.n);
     case kMatPhong:
       if (dot(h.d, n) > 0.f) n = -n;
       if (sx < m.rho_d) {
@@ -361,16 +380,8 @@ __device__ __forceinline__ V3f out_direction(const DeviceScene& S, const Vertex&
       pdf = 1.f;
       V3f d = normalize(h.d);
       float ratio;
-      if (dot(-n, d) < 0.f) { n = -n; ratio = m.ior; } else { ratio = 1.f / m.ior; }
-      float cosI = dot(-n, d);
-      float s2 = fmaxf(0.f, 1.f - cosI * cosI);
-      float sinO = ratio * sqrtf(s2);
-      float cosO = sqrtf(fmaxf(0.f, 1.f - ratio * ratio * s2));
-      float rPerp = (cosI - ratio * cosO) / (cosI + ratio * cosO);
-      float rPara = (ratio * cosI - cosO) / (ratio * cosI + cosO);
-      float R = 0.5f * (rPerp * rPerp + rPara * rPara);
-      if (sinO > 1.f || sx < R) return reflect(d, n);
-      return ratio * d + (ratio * cosI - float(signum(cosI)) * cosO) * n;
+      if (dot_split(-n, d) < 0.f) { n = -n; ratio = m.ior; } else { ratio = 1.f / m.ior; }
+      return refract_or_reflect(d, n, ratio, sx);
     }
     default:
       return v3(0.f, 0.f, 0.f);
@@ -378,7 +389,7 @@ __device__ __forceinline__ V3f out_direction(const DeviceScene& S, const Vertex&
   V3f out = cosine_power_dir(axis, sx, sy, e, pdf);
   if (type == kMatBlinn) {
     const V3f wh = out;
-    const float oh = dot_fused_yx(wo, wh);
+    const float oh = dot_split(wo, wh);
     if (oh < 0.f) { pdf = 0.f; return v3(0.f, 0.f, 0.f); }
     out = v3(__fmaf_rn(2.f * oh, wh.x, -wo.x), __fmaf_rn(2.f * oh, wh.y, -wo.y), __fmaf_rn(2.f * oh, wh.z, -wo.z));
     pdf /= 4.f * fmaxf(oh, 0.0001f);
@@ -479,7 +490,7 @@ __device__ __forceinline__ float env_pdf(const DeviceScene& S, V3f d) {
     u = atan2f(d.x, -d.z) * (0.5f * kInvPi) + 0.5f;
     const float yc = fminf(1.f, fmaxf(-1.f, d.y));
     v = acosf(yc) * kInvPi;
-    jac = (2.f * kPiF * kPiF) * sqrtf(fmaxf(0.f, 1.f - yc * yc));
+    jac = (2.f * kPiF * kPiF) * sqrtf(fmaxf(0.f, __fmaf_rn(-yc, yc, 1.f)));
   } else {
     const float th = acosf(fminf(1.f, fmaxf(-1.f, d.x)));
     const float q = sqrtf(d.y * d.y + d.z * d.z);
@@ -576,18 +587,18 @@ __device__ __forceinline__ V3f phys_eval(const PhysBsdf& b, V3f n, V3f wo, V3f w
     return diff;
   }
   if (b.kind == 2) {
-    V3f r = (2.f * co) * n - wo;
+    V3f r = madv(2.f * co, n, -wo);
     float ca = fmaxf(0.f, dot(r, wi));
     float sp = (b.e + 2.f) * (0.5f * kInvPi) * pow_shared(ca, b.e);
-    pdf = b.pd * ci * kInvPi + (1.f - b.pd) * cos_power_pdf(ca, b.e);
-    return diff + sp * b.ks;
+    pdf = mad2<0>(b.pd * ci, kInvPi, 1.f - b.pd, cos_power_pdf(ca, b.e));
+    return madv(sp, b.ks, diff);
   }
   V3f h = normalize(wi + wo);
   float nh = dot(n, h), oh = dot(wo, h);
   float D = (b.e + 2.f) * (0.5f * kInvPi) * pow_shared(fmaxf(nh, 0.f), b.e);
   float G = fminf(1.f, fminf(2.f * nh * co / oh, 2.f * nh * ci / oh));
-  pdf = b.pd * ci * kInvPi + (1.f - b.pd) * (oh > 0.f ? cos_power_pdf(nh, b.e) / (4.f * oh) : 0.f);
-  return diff + (D * G / (4.f * ci * co)) * b.ks;
+  pdf = mad2<0>(b.pd * ci, kInvPi, 1.f - b.pd, oh > 0.f ? cos_power_pdf(nh, b.e) / (4.f * oh) : 0.f);
+  return madv(D * G / (4.f * ci * co), b.ks, diff);
 }
 
 // Samples wi; weight = f * |cos| / pdf (1 for the specular kinds).
@@ -596,24 +607,14 @@ __device__ __forceinline__ bool phys_sample(const PhysBsdf& b, V3f n, V3f wo, bo
   specular = false;
   pdf = 0.f;
   if (b.kind == 4) {
-    wi = (2.f * dot(n, wo)) * n - wo;
+    wi = madv(2.f * dotf<1>(n, wo), n, -wo);
     specular = true; weight = v3(1.f, 1.f, 1.f); pdf = 1.f;
     return true;
   }
   if (b.kind == 5) {
     // Leaving the medium the geometric normal points along the ray
     // (TransparentMaterial's test, src/transparentmaterial.cpp:43-51).
-    V3f d = -wo;
-    float ratio = exiting ? b.ior : 1.f / b.ior;
-    float cosI = dot(-n, d);
-    float s2 = fmaxf(0.f, 1.f - cosI * cosI);
-    float sinO = ratio * sqrtf(s2);
-    float cosO = sqrtf(fmaxf(0.f, 1.f - ratio * ratio * s2));
-    float rPerp = (cosI - ratio * cosO) / (cosI + ratio * cosO);
-    float rPara = (ratio * cosI - cosO) / (ratio * cosI + cosO);
-    float R = 0.5f * (rPerp * rPerp + rPara * rPara);
-    if (sinO > 1.f || u0 < R) wi = reflect(d, n);
-    else wi = ratio * d + (ratio * cosI - float(signum(cosI)) * cosO) * n;
+    wi = refract_or_reflect(-wo, n, exiting ? b.ior : 1.f / b.ior, u0);
     specular = true; weight = v3(1.f, 1.f, 1.f); pdf = 1.f;
     return true;
   }
@@ -621,23 +622,23 @@ __device__ __forceinline__ bool phys_sample(const PhysBsdf& b, V3f n, V3f wo, bo
   // The lobes choose the axis and the exponent of one cosine-power sample.
   const int lobe = (b.kind == 1 || u0 < b.pd) ? 1 : b.kind;
   V3f axis = n;
-  if (lobe == 2) axis = (2.f * dot(n, wo)) * n - wo;
+  if (lobe == 2) axis = madv(2.f * dotf<1>(n, wo), n, -wo);
   float tmp;
   wi = cosine_power_dir(axis, u1, u2, lobe == 1 ? 1.f : b.e, tmp);
-  if (lobe == 3) wi = (2.f * dot(wo, wi)) * wi - wo;
+  if (lobe == 3) wi = madv(2.f * dotf<1>(wo, wi), wi, -wo);
   V3f f = phys_eval(b, n, wo, wi, pdf);
   if (!(pdf > 0.f)) return false;
   weight = (dot(n, wi) / pdf) * f;
   return true;
 }
 
-__device__ __forceinline__ float power_heuristic(float a, float b) { return a * a / (a * a + b * b); }
+__device__ __forceinline__ float power_heuristic(float a, float b) { return a * a / mad2<0>(a, a, b, b); }
 
 // Uniform direction on the sphere (Sample::getUniformSphereDirection,
 // src/sampler.cpp:78-86).
 __device__ __forceinline__ V3f uniform_sphere(float ux, float uy) {
   float z = 2.f * ux - 1.f;
-  float f = sqrtf(fmaxf(0.f, 1.f - z * z));
+  float f = sqrtf(fmaxf(0.f, __fmaf_rn(-z, z, 1.f)));
   float sn, cs;
   sincospif(2.f * uy, &sn, &cs);
   return v3(f * cs, f * sn, z);
