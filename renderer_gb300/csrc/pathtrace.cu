@@ -278,14 +278,40 @@ __device__ __forceinline__ void warp_add_counters(TraceCounters c, unsigned long
 
 // ----------------------------------------------------- extend / shadow ----
 // Persistent traversal kernels: each warp takes 32 rays at a time from its
-// queue with one atomic and traces them to completion.
+// queue with one atomic and traces them to completion, or, for deep trees
+// (refill_scene), takes new rays for its idle lanes while others still trace.
 //
 // Queue protocol (no host-side resets inside a batch): k_raygen sets
 // counts[0] and zeroes work[0]; k_extend on queue cur zeroes, before shade and
 // shadow run, counts[cur^1] (next extension queue), counts[2] (shadow queue),
 // work[cur^1] (next extend) and work[2] (this iteration's shadow pass).
+
+// Idle lanes of a warp take the queue's next rays. After a bounce the lengths
+// of a warp's rays differ by several times (five to eight of 32 lanes at work
+// on average in a 1.3M-triangle mesh), so a warp with twenty idle lanes refills
+// them. Sooner, a warp waits for new rays and mixes old and new ones more often
+// than its fuller lanes give back; later, lanes idle. Icosphere frame of 67M
+// paths 43.3 ms without, 41.6 / 40.3 / 39.8 with 28 / 24 / 20 idle lanes (in an
+// earlier form 40.4 / 44.5 / 62.6 with 16 / 8 / 1); two rooms 4.58 without,
+// 4.51 / 4.35 / 4.26. Once the queue is empty the lanes finish by themselves:
+// voting at every step makes the longest ray of a launch later (30 us a bounce).
+constexpr int kRefillIdle = 20;
+
+// The index of the ray that this lane takes, -1: none. All lanes call it with
+// the mask of the idle ones.
+__device__ __forceinline__ int refill(unsigned idle, unsigned long long* work, int n, bool& more) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(work, (unsigned long long)__popc(idle));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (base + __popc(idle) >= (unsigned long long)n) more = false;
+  const unsigned long long k = base + __popc(idle & ((1u << lane) - 1u));
+  return (idle >> lane & 1u) && k < (unsigned long long)n ? int(k) : -1;
+}
+
 // MS: the scene of each ray is its job's (gbrt_render_batch_fused).
-template <bool COUNT, bool WT, int STACK, bool GEN, bool MS>
+// REFILL: idle lanes refilled.
+template <bool COUNT, bool WT, int STACK, bool GEN, bool MS, bool REFILL>
 __device__ __forceinline__ void extend_body(const DeviceScene& S, const PTState& st, int cur, const BatchDev& bt) {
   const int n = st.counts[3] ? 0 : st.counts[cur];  // k_finish may have run the last paths
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -298,6 +324,49 @@ __device__ __forceinline__ void extend_body(const DeviceScene& S, const PTState&
   }
   const float4* rays = st.ext[cur];
   unsigned long long* work = st.work + cur;
+  if constexpr (REFILL) {
+    static_assert(!COUNT && !GEN, "refilled rays carry neither counters nor an instance");
+    const DeviceScene* Sp = &S;
+    TState ts;
+    TRay r;
+    int stack[STACK];
+    int i = -1;  // the lane's ray
+    bool more = true;
+    auto store = [&] {
+      RawHit h;
+      h.rec = ts.best;
+      h.t = ts.found ? ts.tcur : CUDART_NAN_F;
+      h.u = ts.bu;
+      h.v = ts.bv;
+      st.hits[i] = h;
+    };
+    for (;;) {
+      const unsigned idle = __ballot_sync(0xffffffffu, i < 0);
+      bool done = false;
+      if (more && __popc(idle) >= kRefillIdle) {
+        const int k = refill(idle, work, n, more);
+        if (k >= 0) {
+          i = k;
+          r = make_tray(rays[2 * i], rays[2 * i + 1]);
+          if (MS) Sp = &bt.scenes[bt.job_of[st.ext_slot[cur][i]]];
+          done = trace_init<false>(MS ? *Sp : S, r, -1, ts);
+        }
+      }
+      if (!more) {
+        if (i < 0) return;
+        while (!done) done = trace_step<false, COUNT, WT, STACK, GEN>(MS ? *Sp : S, r, r, -1, ts, stack, st.err, nullptr);
+        store();
+        return;
+      }
+      if (i >= 0) {
+        if (!done) done = trace_step<false, COUNT, WT, STACK, GEN>(MS ? *Sp : S, r, r, -1, ts, stack, st.err, nullptr);
+        if (done) {
+          store();
+          i = -1;
+        }
+      }
+    }
+  }
   const int lane = threadIdx.x & 31;
   TraceCounters cnt{0, 0};
   for (;;) {
@@ -324,21 +393,67 @@ __device__ __forceinline__ void extend_body(const DeviceScene& S, const PTState&
   if (COUNT) warp_add_counters(cnt, &st.tally[3], &st.tally[4]);
 }
 
-template <bool COUNT, bool WT, int STACK, bool GEN>
+template <bool COUNT, bool WT, int STACK, bool GEN, bool REFILL = false>
 __global__ void __launch_bounds__(kTraceBlock) k_extend(DeviceScene S, PTState st, int cur) {
-  extend_body<COUNT, WT, STACK, GEN, false>(S, st, cur, BatchDev{});
+  extend_body<COUNT, WT, STACK, GEN, false, REFILL>(S, st, cur, BatchDev{});
 }
 
-template <bool WT, int STACK, bool GEN>
+template <bool WT, int STACK, bool GEN, bool REFILL = false>
 __global__ void __launch_bounds__(kTraceBlock) k_extend_ms(PTState st, int cur, BatchDev bt) {
-  extend_body<false, WT, STACK, GEN, true>(bt.scenes[0], st, cur, bt);
+  extend_body<false, WT, STACK, GEN, true, REFILL>(bt.scenes[0], st, cur, bt);
 }
 
-template <bool COUNT, bool WT, int STACK, bool GEN, bool MS>
+template <bool COUNT, bool WT, int STACK, bool GEN, bool MS, bool REFILL>
 __device__ __forceinline__ void shadow_body(const DeviceScene& S, const PTState& st, const BatchDev& bt) {
   const int n = st.counts[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) st.tally[1] += (unsigned long long)n;
   unsigned long long* work = st.work + 2;
+  if constexpr (REFILL) {
+    static_assert(!COUNT && !GEN, "refilled rays carry neither counters nor an instance");
+    const DeviceScene* Sp = &S;
+    TState ts;
+    TRay r;
+    int stack[STACK];
+    int i = -1, slot = 0, ignore = -1;
+    bool more = true;
+    auto unoccluded = [&] {
+      const float4 c = st.sh_c[i];
+      float4* L = st.L + slot;
+      atomicAdd(&L->x, c.x);
+      atomicAdd(&L->y, c.y);
+      atomicAdd(&L->z, c.z);
+    };
+    for (;;) {
+      const unsigned idle = __ballot_sync(0xffffffffu, i < 0);
+      if (more && __popc(idle) >= kRefillIdle) {
+        const int k = refill(idle, work, n, more);
+        if (k >= 0) {
+          i = k;
+          ignore = __float_as_int(st.sh_c[i].w);
+          r = make_tray(st.sh_ray[2 * i], st.sh_ray[2 * i + 1]);
+          slot = st.sh_slot[i];
+          if (MS) Sp = &bt.scenes[bt.job_of[slot]];
+          if (trace_init<true>(MS ? *Sp : S, r, ignore, ts)) {
+            if (ts.best == -1) unoccluded();
+            i = -1;
+          }
+        }
+      }
+      if (!more) {
+        if (i < 0) return;
+        while (!trace_step<true, COUNT, WT, STACK, GEN>(MS ? *Sp : S, r, r, ignore, ts, stack, st.err, nullptr)) {
+        }
+        if (ts.best == -1) unoccluded();
+        return;
+      }
+      if (i >= 0) {
+        if (trace_step<true, COUNT, WT, STACK, GEN>(MS ? *Sp : S, r, r, ignore, ts, stack, st.err, nullptr)) {
+          if (ts.best == -1) unoccluded();
+          i = -1;
+        }
+      }
+    }
+  }
   const int lane = threadIdx.x & 31;
   TraceCounters cnt{0, 0};
   for (;;) {
@@ -369,14 +484,14 @@ __device__ __forceinline__ void shadow_body(const DeviceScene& S, const PTState&
   if (COUNT) warp_add_counters(cnt, &st.tally[5], &st.tally[6]);
 }
 
-template <bool COUNT, bool WT, int STACK, bool GEN>
+template <bool COUNT, bool WT, int STACK, bool GEN, bool REFILL = false>
 __global__ void __launch_bounds__(kTraceBlock) k_shadow(DeviceScene S, PTState st) {
-  shadow_body<COUNT, WT, STACK, GEN, false>(S, st, BatchDev{});
+  shadow_body<COUNT, WT, STACK, GEN, false, REFILL>(S, st, BatchDev{});
 }
 
-template <bool WT, int STACK, bool GEN>
+template <bool WT, int STACK, bool GEN, bool REFILL = false>
 __global__ void __launch_bounds__(kTraceBlock) k_shadow_ms(PTState st, BatchDev bt) {
-  shadow_body<false, WT, STACK, GEN, true>(bt.scenes[0], st, bt);
+  shadow_body<false, WT, STACK, GEN, true, REFILL>(bt.scenes[0], st, bt);
 }
 
 // What the error word of a render says (bits kErrStack, kErrIndex).
@@ -1424,6 +1539,8 @@ static CamDev make_camera(const gbrt_camera& c) {
 struct TraceKernels {
   void (*ext)(DeviceScene, PTState, int);
   void (*sh)(DeviceScene, PTState);
+  void (*camera)(DeviceScene, PTState, int) = nullptr;  // camera rays, null: ext
+  void (*extend(int it) const)(DeviceScene, PTState, int) { return it == 0 && camera ? camera : ext; }
 };
 template <bool C, bool W, bool G>
 static TraceKernels pick_stack(bool shortStack) {
@@ -1435,6 +1552,22 @@ static TraceKernels pick_flags(bool count, bool wt, bool shortStack) {
   if (count) return wt ? pick_stack<true, true, G>(shortStack) : pick_stack<true, false, G>(shortStack);
   return wt ? pick_stack<false, true, G>(shortStack) : pick_stack<false, false, G>(shortStack);
 }
+// Whether the traversal kernels refill idle lanes: trees of eight levels and
+// more, where rays are long and of different lengths. Without / with, 4.2M paths
+// into the icosphere of 4 / 5 / 6 / 7 subdivisions (8 to 11 levels): 2585 / 2582,
+// 2927 / 2887, 3345 / 3279, 3861 / 3685 us; of 1 to 3 (4 to 6 levels): 2008 /
+// 2076, 2141 / 2217, 2329 / 2370; two rooms of 4 / 6 / 8 / 10 levels: 3061 /
+// 3297, 3579 / 3567, 4327 / 4127, 5107 / 4752. Camera rays stay together and are
+// traced 32 at a time in any tree (rooms of 10 levels 4850 otherwise). Scenes
+// with instances or CSG objects keep the plain kernels: the refilled ones spill
+// there (terrain 3.64 ms plain, 3.73 refilled).
+constexpr int kRefillDepth = 8;
+
+static bool refill_scene(const gbrt_scene* s) {
+  return s->max_depth4 >= kRefillDepth && stack_need(s->max_depth4) <= kShortStack && !s->watertight &&
+         !s->view.csg_prog && !s->view.inst;
+}
+
 // Traversal counters, watertight triangles, short stack when the tree is
 // shallow enough, the general leaves (CSG objects, instances) only for scenes
 // that have them.
@@ -1447,6 +1580,8 @@ static TraceKernels pick_kernels(const gbrt_scene* s, bool count) {
   }
   const bool shortStack = stack_need(s->max_depth4) <= kShortStack;
   if (s->view.csg_prog || s->view.inst) return pick_flags<true>(count, s->watertight, shortStack);
+  if (!count && refill_scene(s)) return {k_extend<false, false, kShortStack, false, true>, k_shadow<false, false, kShortStack, false, true>,
+            k_extend<false, false, kShortStack, false>};
   return pick_flags<false>(count, s->watertight, shortStack);
 }
 
@@ -1622,11 +1757,10 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render set-up");
 
   const TraceKernels tk = pick_kernels(s, count);
-  auto kExt = tk.ext;
   auto kSh = tk.sh;
   // Persistent grids: every SM filled with as many blocks as fit.
   int per = 0;
-  if (!whole) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kExt, kTraceBlock, 0);
+  if (!whole) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tk.ext, kTraceBlock, 0);
   const int traceGrid = std::max(1, per) * ctx->num_sms;
   if (!whole) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kSh, kTraceBlock, 0);
   const int shadowGrid = std::max(1, per) * ctx->num_sms;
@@ -1663,7 +1797,7 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
           ++launches;
         }
         if (timeK) mark();
-        kExt<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+        tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
         if (timeK) mark();
         kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
         if (timeK) mark();
@@ -1846,10 +1980,9 @@ static gbrt_status render_noalloc_impl(gbrt_scene* s, const gbrt_camera* cam, co
   if (e != cudaSuccess) return cuda_fail(ctx, e, "gbrt_render_device_noalloc set-up");
 
   const TraceKernels tk = pick_kernels(s, (prm->flags & GBRT_RENDER_COUNT_TRAVERSAL) != 0);
-  auto kExt = tk.ext;
   auto kSh = tk.sh;
   int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kExt, kTraceBlock, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, tk.ext, kTraceBlock, 0);
   const int traceGrid = std::max(1, per) * ctx->num_sms;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kSh, kTraceBlock, 0);
   const int shadowGrid = std::max(1, per) * ctx->num_sms;
@@ -1870,7 +2003,7 @@ static gbrt_status render_noalloc_impl(gbrt_scene* s, const gbrt_camera* cam, co
       ++launches;
       for (int it = 0; it < P.D; ++it) {
         int cur = it & 1;
-        kExt<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+        tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
         kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
         kSh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
         launches += 3;
@@ -2199,7 +2332,7 @@ static gbrt_status render_guided_impl(gbrt_scene* s, const gbrt_camera* cam, con
         for (int it = 0; it < P.D; ++it) {
           int cur = it & 1;
           if (pk.finish && it >= kFinishFrom) launch_finish(pk, s, P, st, cur, stream);
-          tk.ext<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+          tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
           if (P.guided && (P.guide_depth == 0 || it < P.guide_depth)) {
             cudaEvent_t ea = nullptr, eb = nullptr;
             if (timeK) {
@@ -2402,7 +2535,7 @@ static cudaError_t enqueue_job(gbrt_scene* s, const gbrt_camera& cam, const gbrt
     k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
     for (int it = 0; it < P.D; ++it) {
       int cur = it & 1;
-      tk.ext<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
+      tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
       kShade<<<cap_grid(shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
       tk.sh<<<cap_grid(shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
     }
@@ -2533,20 +2666,22 @@ static gbrt_status batch_impl(gbrt_ctx* ctx, const gbrt_batch_job* jobs, int n, 
 // The fused batch's kernels for the jobs' scenes: the general leaves if any
 // scene needs them, the short stack only if every tree is shallow enough.
 struct FusedKernels {
+  void (*camera)(PTState, int, BatchDev);  // extends camera rays
   void (*ext)(PTState, int, BatchDev);
   void (*sh)(PTState, BatchDev);
   void (*shade)(PTState, int, BatchDev);
 };
-template <bool W, int K, bool G>
+template <bool W, int K, bool G, bool R = false>
 static FusedKernels fused_trace(bool physical, bool ext) {
-  FusedKernels f{k_extend_ms<W, K, G>, k_shadow_ms<W, K, G>, nullptr};
+  FusedKernels f{k_extend_ms<W, K, G>, k_extend_ms<W, K, G, R>, k_shadow_ms<W, K, G, R>, nullptr};
   if (physical) f.shade = ext ? k_shade_phys_ms<true> : k_shade_phys_ms<false>;
   else f.shade = ext ? k_shade_ms<true> : k_shade_ms<false>;
   return f;
 }
 template <bool W>
-static FusedKernels fused_pick(bool shortStack, bool gen, bool physical, bool ext) {
+static FusedKernels fused_pick(bool shortStack, bool gen, bool refill, bool physical, bool ext) {
   if (gen) return shortStack ? fused_trace<W, kShortStack, true>(physical, ext) : fused_trace<W, kStackSize, true>(physical, ext);
+  if (!W && refill) return fused_trace<false, kShortStack, false, true>(physical, ext);
   return shortStack ? fused_trace<W, kShortStack, false>(physical, ext) : fused_trace<W, kStackSize, false>(physical, ext);
 }
 
@@ -2576,7 +2711,7 @@ static gbrt_status batch_fused_impl(gbrt_ctx* ctx, const gbrt_batch_job* jobs, i
   if (B < 1) return fail(ctx, GBRT_ERR_INVALID_ARG, "gbrt_render_batch_fused: wavefront size");
   const bool physical = jobs[0].params.semantics == GBRT_SEM_PHYSICAL;
   const bool wt = jobs[0].scene->watertight;
-  bool gen = false, ext = false, shortStack = true, anyInst = false;
+  bool gen = false, ext = false, shortStack = true, anyInst = false, deep = false;
   int D = 0;
   unsigned long long total = 0, pixels = 0;
   // The jobs are numbered smallest first (paths x depth), so that small
@@ -2604,6 +2739,7 @@ static gbrt_status batch_fused_impl(gbrt_ctx* ctx, const gbrt_batch_job* jobs, i
     anyInst = anyInst || scn->view.inst;
     ext = ext || ext_scene(scn);
     shortStack = shortStack && stack_need(scn->max_depth4) <= kShortStack;
+    deep = deep || scn->max_depth4 >= kRefillDepth;
     D = std::max(D, jb.params.max_depth);
     const unsigned long long np = (unsigned long long)jb.camera.width * jb.camera.height;
     const unsigned long long tj = np * (unsigned long long)(jb.params.x_samples * jb.params.y_samples);
@@ -2688,8 +2824,9 @@ static gbrt_status batch_fused_impl(gbrt_ctx* ctx, const gbrt_batch_job* jobs, i
   A(cudaStreamSynchronize(stream));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "gbrt_render_batch_fused set-up");
 
-  const FusedKernels fk = wt ? fused_pick<true>(shortStack, gen, physical, ext)
-                             : fused_pick<false>(shortStack, gen, physical, ext);
+  const bool refill = deep && shortStack;  // any deep tree: its rays are the long ones
+  const FusedKernels fk = wt ? fused_pick<true>(shortStack, gen, refill, physical, ext)
+                             : fused_pick<false>(shortStack, gen, refill, physical, ext);
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fk.ext, traceBlock, 0);
   const int traceGrid = std::max(1, per) * ctx->num_sms;
@@ -2712,7 +2849,7 @@ static gbrt_status batch_fused_impl(gbrt_ctx* ctx, const gbrt_batch_job* jobs, i
     k_raygen_ms<<<unsigned((B + 255) / 256), 256, 0, q>>>(st, bt);
     for (int it = 0; it < D; ++it) {
       const int cur = it & 1;
-      fk.ext<<<cap_grid(traceGrid, B, traceBlock), traceBlock, 0, q>>>(st, cur, bt);
+      (it == 0 ? fk.camera : fk.ext)<<<cap_grid(traceGrid, B, traceBlock), traceBlock, 0, q>>>(st, cur, bt);
       fk.shade<<<cap_grid(shadeGrid, B, shadeBlock), shadeBlock, 0, q>>>(st, cur, bt);
       fk.sh<<<cap_grid(shadowGrid, 2 * B, traceBlock), traceBlock, 0, q>>>(st, bt);
     }
