@@ -687,6 +687,35 @@ gbrt_status read_err(gbrt_guide* g, cudaStream_t stream) {
   return GBRT_OK;
 }
 
+// The rows of the C ABI (9 floats an input, 13 a sample, 40 a mixture) to and
+// from the kernels' 16-byte columns, one column a thread. On the host this was
+// most of a call: a first touch of the repacked copy's pages, and a strided copy
+// of the mixtures back (200,000-row evaluations and sample steps of 2^18 rows,
+// through the C ABI: 2.3-2.7 -> 1.07 ms and 1.42 -> 0.33 ms).
+// IN floats a row: three at a time; the first column's fourth is the row's last
+// float when there is one (a sample's radiance estimate).
+template <int IN, int COLS>
+__global__ void __launch_bounds__(256) k_pack_rows(const float* __restrict__ in, unsigned n, float4* __restrict__ out) {
+  const unsigned j = blockIdx.x * 256u + threadIdx.x;
+  if (j >= COLS * n) return;
+  const unsigned row = j / COLS, c = j - row * COLS;
+  const float* r = in + size_t(row) * IN + 3 * c;
+  out[j] = make_float4(r[0], r[1], r[2], IN > 3 * COLS && c == 0 ? r[3 * COLS] : 0.f);
+}
+
+__global__ void __launch_bounds__(256) k_pack_mixtures(const float4* __restrict__ mix, unsigned n,
+                                                       float4* __restrict__ out) {
+  const unsigned j = blockIdx.x * 256u + threadIdx.x;
+  if (j >= 10u * n) return;
+  const unsigned row = j / 10u;
+  out[j] = mix[size_t(row) * kMixStride + (j - row * 10u)];
+}
+
+constexpr int kMixFloats = 40;
+// Rows of gbrt_guide_eval in flight: bounds its workspace to 450 MB; a million
+// rows fill the GPU many times.
+constexpr size_t kEvalRows = size_t(1) << 20;
+
 }  // namespace
 
 extern "C" {
@@ -808,41 +837,52 @@ gbrt_status gbrt_guide_eval(gbrt_guide* g, const float* inputs, size_t n, float*
   if (n == 0) return GBRT_OK;
   if (n > (1u << 26)) return fail(g->ctx, GBRT_ERR_INVALID_ARG, "gbrt_guide_eval: too many rows");
   cudaStream_t s = g->ctx->stream;
-  std::vector<float4> h(3 * n);
-  for (size_t i = 0; i < n; ++i) {
-    const float* r = inputs + 9 * i;
-    h[3 * i] = make_float4(r[0], r[1], r[2], 0.f);
-    h[3 * i + 1] = make_float4(r[3], r[4], r[5], 0.f);
-    h[3 * i + 2] = make_float4(r[6], r[7], r[8], 0.f);
-  }
+  const size_t rows = std::min(n, kEvalRows);
+  float *d_raw = nullptr, *d_res = nullptr;
   float4 *d_in = nullptr, *d_mix = nullptr;
-  cudaError_t e = ctx_alloc(g->ctx, &d_in, h.size() * sizeof(float4), s);
-  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_mix, kMixStride * n * sizeof(float4), s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = launch_infer(g, d_in, nullptr, int(n), d_mix, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpy2DAsync(out, 10 * sizeof(float4), d_mix, kMixStride * sizeof(float4), 10 * sizeof(float4), n,
-                          cudaMemcpyDeviceToHost, s);
+  cudaError_t e = ctx_alloc(g->ctx, &d_raw, rows * 9 * sizeof(float), s);
+  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_in, rows * 3 * sizeof(float4), s);
+  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_mix, rows * kMixStride * sizeof(float4), s);
+  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_res, rows * kMixFloats * sizeof(float), s);
+  for (size_t i = 0; i < n && e == cudaSuccess; i += rows) {
+    const size_t m = std::min(rows, n - i);
+    e = cudaMemcpyAsync(d_raw, inputs + 9 * i, m * 9 * sizeof(float), cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) break;
+    k_pack_rows<9, 3><<<unsigned((3 * m + 255) / 256), 256, 0, s>>>(d_raw, unsigned(m), d_in);
+    e = launch_infer(g, d_in, nullptr, int(m), d_mix, s);
+    if (e != cudaSuccess) break;
+    k_pack_mixtures<<<unsigned((10 * m + 255) / 256), 256, 0, s>>>(d_mix, unsigned(m),
+                                                                    reinterpret_cast<float4*>(d_res));
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out + kMixFloats * i, d_res, m * kMixFloats * sizeof(float), cudaMemcpyDeviceToHost, s);
+  }
+  if (d_raw) cudaFreeAsync(d_raw, s);
   if (d_in) cudaFreeAsync(d_in, s);
   if (d_mix) cudaFreeAsync(d_mix, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (d_res) cudaFreeAsync(d_res, s);
+  const cudaError_t f = cudaStreamSynchronize(s);  // after an error too: the copies use the caller's memory
+  if (e == cudaSuccess) e = f;
   if (e != cudaSuccess) return cuda_fail(g->ctx, e, "gbrt_guide_eval");
   return read_err(g, s);
 }
 
 static gbrt_status upload_samples(gbrt_guide* g, const float* samples, size_t n, float4** d_out) {
-  std::vector<float4> h(4 * n);
-  for (size_t i = 0; i < n; ++i) {
-    const float* r = samples + 13 * i;
-    h[4 * i] = make_float4(r[0], r[1], r[2], r[12]);
-    h[4 * i + 1] = make_float4(r[3], r[4], r[5], 0.f);
-    h[4 * i + 2] = make_float4(r[6], r[7], r[8], 0.f);
-    h[4 * i + 3] = make_float4(r[9], r[10], r[11], 0.f);
-  }
   cudaStream_t s = g->ctx->stream;
-  cudaError_t e = ctx_alloc(g->ctx, d_out, h.size() * sizeof(float4), s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(*d_out, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  float* d_raw = nullptr;
+  cudaError_t e = ctx_alloc(g->ctx, d_out, n * 4 * sizeof(float4), s);
+  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_raw, n * 13 * sizeof(float), s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_raw, samples, n * 13 * sizeof(float), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) {
+    k_pack_rows<13, 4><<<unsigned((4 * n + 255) / 256), 256, 0, s>>>(d_raw, unsigned(n), *d_out);
+    e = cudaGetLastError();
+  }
+  if (d_raw) cudaFreeAsync(d_raw, s);
+  if (e != cudaSuccess) {
+    if (*d_out) cudaFreeAsync(*d_out, s);
+    *d_out = nullptr;
+    cudaStreamSynchronize(s);  // the copy uses the caller's memory
+  }
   if (e != cudaSuccess) return cuda_fail(g->ctx, e, "guide samples");
   return GBRT_OK;
 }
@@ -860,7 +900,8 @@ gbrt_status gbrt_guide_gradient(gbrt_guide* g, const float* samples, size_t n, f
   float l = 0.f;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&l, g->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(d, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  const cudaError_t f = cudaStreamSynchronize(s);  // after an error too, as in gbrt_guide_eval
+  if (e == cudaSuccess) e = f;
   if (e != cudaSuccess) return cuda_fail(g->ctx, e, "gbrt_guide_gradient");
   if (loss) *loss = l;
   return read_err(g, s);
@@ -878,7 +919,8 @@ gbrt_status gbrt_guide_train_step(gbrt_guide* g, const float* samples, size_t n,
   float l = 0.f;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&l, g->d_loss, sizeof(float), cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(d, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  const cudaError_t f = cudaStreamSynchronize(s);  // after an error too, as in gbrt_guide_eval
+  if (e == cudaSuccess) e = f;
   if (e != cudaSuccess) return cuda_fail(g->ctx, e, "gbrt_guide_train_step");
   if (loss) *loss = l;
   return read_err(g, s);
