@@ -53,6 +53,8 @@ constexpr int kInferWG = 6;
 constexpr int kEncA = 14, kEncB = 12;  // groups of 8 features in the two halves
 constexpr int kInferBuf = kRows * kEncA * 8 * 2;
 constexpr int kInferMisc = kSWEnd + kInferWG * kInferBuf, kInferSmem = kInferMisc + 8 * kInferWG + 16;
+constexpr int kStageRow = 16 * kMixStride + 16;  // odd in 16-byte units: rows start in different banks
+static_assert(kRows * kStageRow <= kInferBuf, "a tile's mixtures fit its rows' buffer");
 constexpr uint32_t kInferCols = 512;  // 64 per warpgroup, rounded up to a power of two
 
 // Training: the weights, the activation rows X1..X3, the region R (the
@@ -143,6 +145,12 @@ __global__ void __launch_bounds__(128 * kInferWG, 1) k_guide_infer(GuideNet net,
   const uint32_t sW1 = smem_u32(sm + kSW1), sW2 = smem_u32(sm + kSW2), sW3 = smem_u32(sm + kSW3),
                  sW4 = smem_u32(sm + kSW4), sX = smem_u32(sm + kSWEnd + wg * kInferBuf), bar = smem_u32(mbar);
   const int bid = 1 + wg;  // named barrier of this warpgroup
+  // The mixtures of a warp's 32 rows on their way out: a lane's own row is 192
+  // bytes, so storing it from registers spread each instruction over 32 rows
+  // (four times the bytes on the way to L2). Rewritten in shared memory, 32
+  // lanes store 512 consecutive bytes: 800,000 rows 116 -> 94 us, the guided
+  // passes 6.11 -> 5.82 ms. (Fetching the next tile's inputs early: no gain.)
+  uint8_t* stage = sm + kSWEnd + wg * kInferBuf + (warp & 3) * 32 * kStageRow;
   load_weights(sm + kSW1, net.w + kOffW1, kHid, kIn, kHid);
   load_weights(sm + kSW2, net.w + kOffW2, kHid, kHid, kHid);
   load_weights(sm + kSW3, net.w + kOffW3, kHid, kHid, kHid);
@@ -210,8 +218,13 @@ __global__ void __launch_bounds__(128 * kInferWG, 1) k_guide_infer(GuideNet net,
         if (r < n) {
           Mixture m;
           decode_mixture(o, m);
-          store_mixture(mix + kMixStride * size_t(r), m);
+          store_mixture(reinterpret_cast<float4*>(stage + kStageRow * (t & 31)), m);
         }
+        __syncwarp();
+        const int first = r & ~31, have = min(32, n - first) * kMixStride;
+        float4* out = mix + kMixStride * size_t(first);
+        for (int j = t & 31; j < have; j += 32)
+          out[j] = *reinterpret_cast<const float4*>(stage + kStageRow * (j / kMixStride) + 16 * (j % kMixStride));
       }
     }
     if (!ok) break;
