@@ -1095,8 +1095,8 @@ def main():
                 "fetched_bytes_per_ray": fetched_per_ray,
                 "frac_fetched": tot["ext_rays"] * fetched_per_ray / ext_s / 1e9 / peak,
                 "bound_note": "issue- and divergence-bound, not bandwidth-bound: nodes and records come mostly "
-                              "from L1/L2 (dram_frac is what DRAM carries); ncu: 72-75 % issue-active, 21 of 32 "
-                              "lanes active on camera rays and 9 on bounces (profiles/k_extend_icosphere.md)",
+                              "from L1/L2 (dram_frac is what DRAM carries); ncu: 65-72 % issue-active, 16-21 "
+                              "of 32 lanes active on camera rays, idle lanes refilled on bounces",
                 "launches": tot["ext_launch"], "avg_launch_ms": 1000.0 * avg_launch_s,
                 "share_of_render": tot["ext_ms"] / max(tot["ms"], 1e-9)}
 
