@@ -124,7 +124,7 @@ struct DeviceScene {
   // Textures (null when no material uses one): texels of all textures one
   // after the other (3 floats, BGR), per texture (first texel, W, H, -), and
   // per triangle its three texture coordinates (6 floats, input order; the
-  // triangle of primitive id p is p - tri_pid0).
+  // triangle of primitive id p is p - tri_pid0; null also without triangles).
   const float* tex_texels;
   const int4* tex_info;
   const float* tri_uv;

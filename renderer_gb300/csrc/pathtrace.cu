@@ -675,7 +675,7 @@ __device__ __forceinline__ void shade_vertex(const DeviceScene& S, const PTParam
       vx.mat = m.y;
       light = m.w;
       if (!in_range(light < S.n_lights && vx.mat < S.n_materials, err)) return;
-      if (EXT && S.tri_uv) hit_texcoords(S, h.rec, h.u, h.v, vx.p, vx.tu, vx.tv);
+      if (EXT && S.tex_info) hit_texcoords(S, h.rec, h.u, h.v, vx.p, vx.tu, vx.tv);
       if (kind == kRecTriangle) {
         if (m.z >= 0) {
           const float* nn = S.tri_nrm + 12 * int64_t(m.z);
@@ -914,7 +914,7 @@ __device__ __forceinline__ void surface_normal(const DeviceScene& S, const RawHi
       nrm = normf<0>(x - v3(a.x, a.y, a.z));  // sphere
     }
     if (EXT && inst >= 0) nrm = instance_normal(S, inst, nrm);
-    if (EXT && S.tri_uv) hit_texcoords(S, h.rec, h.u, h.v, x, tu, tv);
+    if (EXT && S.tex_info) hit_texcoords(S, h.rec, h.u, h.v, x, tu, tv);
   } else {
     const float4 pl = __ldg(&S.planes[-2 - h.rec]);
     nrm = normalize(v3(pl.x, pl.y, pl.z));
@@ -1588,7 +1588,7 @@ static TraceKernels pick_kernels(const gbrt_scene* s, bool count) {
 // The shade kernel: estimator, guiding, and the texture / CSG / instance code
 // only for scenes that have textures, CSG objects or instances.
 static bool ext_scene(const gbrt_scene* s) {
-  return s->view.tri_uv != nullptr || s->view.csg_prog != nullptr || s->view.inst != nullptr;
+  return s->view.tex_info != nullptr || s->view.csg_prog != nullptr || s->view.inst != nullptr;
 }
 static void (*pick_shade(const gbrt_scene* s, bool physical, bool guided))(DeviceScene, PTParams, PTState, int) {
   const bool ext = ext_scene(s);

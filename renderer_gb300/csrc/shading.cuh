@@ -200,7 +200,7 @@ __device__ __forceinline__ void hit_texcoords(const DeviceScene& S, int rec, flo
                                               float& tv) {
   tu = 0.f;
   tv = 0.f;
-  if (!S.tri_uv || rec < 0) return;
+  if (rec < 0) return;
   const float4* rp = S.recs + 3 * int64_t(rec);
   const float4 a = __ldg(rp);
   const int kind = __float_as_int(a.w);
@@ -399,7 +399,7 @@ __device__ __forceinline__ V3f out_direction(const DeviceScene& S, const Vertex&
     brdf = phong_spec(m, h, out);
   } else if (EXT && type == kMatTexture) {
     brdf = kInvPi * texture_albedo(S, m, h.tu, h.tv);
-  } else if (type != kMatTexture) {
+  } else {
     brdf = v3(m.kd[0] * kInvPi, m.kd[1] * kInvPi, m.kd[2] * kInvPi);
   }
   return out;
