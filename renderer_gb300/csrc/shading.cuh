@@ -414,8 +414,10 @@ __device__ __forceinline__ V3f area_intensity(const DevLight& L, V3f dir) {
 }
 
 // EnvironmentMap::get(direction). Angular light probe (+x at the centre) or
-// equirectangular; nearest texel, indices clamped into the image.
-__device__ __forceinline__ int env_texel(int W, int H, int mapping, float x, float y, float z) {
+// equirectangular; nearest texel, indices clamped into the image. A map may
+// have more than 2^31 texels, so the index is 64-bit (__host__: a test calls it
+// for such maps without one in memory).
+__host__ __device__ __forceinline__ size_t env_texel(int W, int H, int mapping, float x, float y, float z) {
   int row, col;
   if (mapping == GBRT_ENV_LATLONG) {
     float u = atan2f(x, -z) * (0.5f * kInvPi) + 0.5f;
@@ -433,10 +435,10 @@ __device__ __forceinline__ int env_texel(int W, int H, int mapping, float x, flo
   }
   row = min(max(row, 0), H - 1);
   col = min(max(col, 0), W - 1);
-  return row * W + col;
+  return size_t(row) * W + col;
 }
 __device__ __forceinline__ V3f env_get(const DeviceScene& S, V3f d) {
-  const float* p = S.env_texels + size_t(env_texel(S.env_w, S.env_h, S.env_mapping, d.x, d.y, d.z)) * 3;
+  const float* p = S.env_texels + env_texel(S.env_w, S.env_h, S.env_mapping, d.x, d.y, d.z) * 3;
   return v3(__ldg(p) * S.env_coef[0], __ldg(p + 1) * S.env_coef[1], __ldg(p + 2) * S.env_coef[2]);
 }
 
