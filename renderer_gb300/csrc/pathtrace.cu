@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(256) k_guide_collect(PTParams P, PTState st) {
   const double* ps = P.film_sum + 3 * pix;
   const double* pc = P.pass_sum + 3 * pix;
   const float pl = float((ps[0] + ps[1] + ps[2] + pc[0] + pc[1] + pc[2]) * (1.0 / 3.0) * P.inv_samples);
-  const float inv_pix = rsqrtf(pl * pl + 0.01f);
+  const float inv_pix = rsqrtf(__fmaf_rn(pl, pl, 0.01f));
   for (int r = 0; r < nrec; ++r) {
     const size_t b = size_t(kRecComp * r) * ns + slot;
     const float4 r0 = st.rec[b], r1 = st.rec[b + ns], r2 = st.rec[b + 2 * ns], r3 = st.rec[b + 3 * ns],
@@ -1253,7 +1253,7 @@ __global__ void __launch_bounds__(256) k_guide_collect(PTParams P, PTState st) {
       if (r3.x > 0.f) li += (L.x - sn.x) / r3.x;
       if (r3.y > 0.f) li += (L.y - sn.y) / r3.y;
       if (r3.z > 0.f) li += (L.z - sn.z) / r3.z;
-      const float cosi = fabsf(r1.x * r1.w + r1.y * r2.w + r1.z * r3.w);
+      const float cosi = fabsf(__fmaf_rn(r1.z, r3.w, mad2<0>(r1.x, r1.w, r1.y, r2.w)));
       w = (li * (1.f / 3.f)) * cosi / r0.w;
     }
     if (P.train_relative) w *= r5.x * inv_pix;
@@ -2058,7 +2058,7 @@ __global__ void __launch_bounds__(256) k_pass_deviation(const double* __restrict
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n3; i += size_t(gridDim.x) * blockDim.x) {
     double x = pass_sum[i] * inv_pass, m = prev_sum[i] * inv_prev;
     double d = x - m;
-    if (isfinite(d)) acc += d * d / (m * m + 0.01);
+    if (isfinite(d)) acc += d * d / __fma_rn(m, m, 0.01);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   __shared__ double part[8];
@@ -2087,7 +2087,7 @@ __global__ void k_pass_combine(const double* __restrict__ pass_sum, double* __re
   if (i >= n3) return;
   double x = pass_sum[i];
   prev_sum[i] += x;
-  if (w > 0.0) weighted[i] += w * x * inv_pass;
+  if (w > 0.0) weighted[i] = __fma_rn(w * x, inv_pass, weighted[i]);
 }
 
 // film = (sum over passes of w * pass mean) / (sum of w).

@@ -159,7 +159,7 @@ __device__ __forceinline__ void csg_surface(const DeviceScene& S, int leaf, V3f 
     const V3f nn = x - v3(A.x, A.y, A.z);
     n = normalize(nn);
     tu = acosf(nn.z / B.x) * kInvPi;
-    tv = atan2f(nn.x, nn.y) * (0.5f * kInvPi) + 0.5f;
+    tv = __fmaf_rn(atan2f(nn.x, nn.y), 0.5f * kInvPi, 0.5f);
     return;
   }
   const float oo[3] = {o.x, o.y, o.z}, dd[3] = {d.x, d.y, d.z};
@@ -208,7 +208,7 @@ __device__ __forceinline__ void hit_texcoords(const DeviceScene& S, int rec, flo
     const float r = __ldg(rp + 1).x;
     const V3f n = x - v3(a.x, a.y, a.z);
     tu = acosf(n.z / r) * kInvPi;
-    tv = atan2f(n.x, n.y) * (0.5f * kInvPi) + 0.5f;
+    tv = __fmaf_rn(atan2f(n.x, n.y), 0.5f * kInvPi, 0.5f);
     return;
   }
   if (kind != kRecTriangle) return;
@@ -258,8 +258,9 @@ __device__ __forceinline__ V3f texture_albedo(const DeviceScene& S, const DevMat
   V3f r;
   float* rr = &r.x;
   for (int c = 0; c < 3; ++c) {
-    float s = __ldg(T + (int64_t(y0) * W + x0) * 3 + c) * w00 + __ldg(T + (int64_t(y0) * W + x1) * 3 + c) * w10 +
-              __ldg(T + (int64_t(y1) * W + x0) * 3 + c) * w01 + __ldg(T + (int64_t(y1) * W + x1) * 3 + c) * w11;
+    float s = mad2<0>(__ldg(T + (int64_t(y0) * W + x0) * 3 + c), w00, __ldg(T + (int64_t(y0) * W + x1) * 3 + c), w10);
+    s = __fmaf_rn(__ldg(T + (int64_t(y1) * W + x0) * 3 + c), w01, s);
+    s = __fmaf_rn(__ldg(T + (int64_t(y1) * W + x1) * 3 + c), w11, s);
     s *= m.kd[c];
     rr[c] = m.exponent == 1.f ? s : pow_shared(s, m.exponent);
   }
@@ -420,16 +421,16 @@ __device__ __forceinline__ V3f area_intensity(const DevLight& L, V3f dir) {
 __host__ __device__ __forceinline__ size_t env_texel(int W, int H, int mapping, float x, float y, float z) {
   int row, col;
   if (mapping == GBRT_ENV_LATLONG) {
-    float u = atan2f(x, -z) * (0.5f * kInvPi) + 0.5f;
+    float u = fmaf(atan2f(x, -z), 0.5f * kInvPi, 0.5f);
     float v = acosf(fminf(1.f, fmaxf(-1.f, y))) * kInvPi;
     col = min(int(u * W), W - 1);
     row = min(int(v * H), H - 1);
   } else {
     float cx = y, cy = -z;
-    float f = acosf(x) / (sqrtf(cx * cx + cy * cy) * CUDART_PI_F);
-    cx *= f; cy *= f;
-    int px = int((cx + 1.f) * 0.5f * float(W) - 1.f);
-    int py = int((cy + 1.f) * 0.5f * float(H) - 1.f);
+    float f = acosf(x) / (sqrtf(fmaf(cy, cy, cx * cx)) * CUDART_PI_F);
+    cx = fmaf(cx, f, 1.f); cy = fmaf(cy, f, 1.f);
+    int px = int(fmaf(cx * 0.5f, float(W), -1.f));
+    int py = int(fmaf(cy * 0.5f, float(H), -1.f));
     row = min(py, W - 1);
     col = min(px, H - 1);
   }
@@ -468,7 +469,7 @@ __device__ __forceinline__ bool env_param_dir(const DeviceScene& S, float u, flo
     jac = (2.f * kPiF * kPiF) * st;
   } else {
     const float cx = 2.f * u - 1.f, cy = 2.f * v - 1.f;
-    const float r = sqrtf(cx * cx + cy * cy);
+    const float r = sqrtf(mad2<1>(cx, cx, cy, cy));
     if (!(r < 1.f)) return false;
     if (r == 0.f) {
       d = v3(1.f, 0.f, 0.f);
@@ -489,16 +490,16 @@ __device__ __forceinline__ float env_pdf(const DeviceScene& S, V3f d) {
   const int W = S.env_w, H = S.env_h;
   float u, v, jac;
   if (S.env_mapping == GBRT_ENV_LATLONG) {
-    u = atan2f(d.x, -d.z) * (0.5f * kInvPi) + 0.5f;
+    u = __fmaf_rn(atan2f(d.x, -d.z), 0.5f * kInvPi, 0.5f);
     const float yc = fminf(1.f, fmaxf(-1.f, d.y));
     v = acosf(yc) * kInvPi;
     jac = (2.f * kPiF * kPiF) * sqrtf(fmaxf(0.f, __fmaf_rn(-yc, yc, 1.f)));
   } else {
     const float th = acosf(fminf(1.f, fmaxf(-1.f, d.x)));
-    const float q = sqrtf(d.y * d.y + d.z * d.z);
+    const float q = sqrtf(mad2<1>(d.y, d.y, d.z, d.z));
     const float f = q > 0.f ? th / (q * kPiF) : 0.f;
-    u = (d.y * f + 1.f) * 0.5f;
-    v = (-d.z * f + 1.f) * 0.5f;
+    u = __fmaf_rn(d.y, f, 1.f) * 0.5f;
+    v = __fmaf_rn(-d.z, f, 1.f) * 0.5f;
     jac = th > 0.f ? (4.f * kPiF * kPiF) * q / th : 4.f * kPiF * kPiF;
   }
   if (!(jac > 0.f)) return 0.f;
