@@ -1626,7 +1626,16 @@ static long long path_lanes(const gbrt_ctx* ctx) { return 512ll * ctx->num_sms; 
 // box (one level) 131k paths 425 / 342, 262k 540 / 588; two rooms of 500,000
 // triangles 262k 1330 / 888, 524k 1729 / 1623; icosphere of 1.31M 262k
 // 2036 / 816, 1M 3132 / 2454.
+// With instances the costs are higher (the ray in two spaces, the CSG code: fewer
+// lanes at work in a bigger kernel) and the line lies lower. Five bounces, by
+// bounces / by k_path, us, at 1 / 2 / 3 paths per lane and above: four meshes in
+// a room (9 levels) 734 / 549 at 65k, 772 / 872 at 102k, 947 / 1797 at 262k; 30
+// meshes (11 levels) 1341 / 1360 at 147k; eight of 20,000 triangles (12 levels)
+// 1328 / 1294 at 147k, 1437 / 1658 at 200k; eight of 327,680 (15 levels)
+// 2216 / 2142 at 262k; an open terrain (15 levels, three bounces) 645 / 637 at
+// 262k. So 2/3 of a path per lane up to eight levels, 1/3 more a level, at most 3.
 static long long whole_path_limit(const gbrt_scene* s) {
+  if (s->view.inst) return path_lanes(s->ctx) * std::min(std::max(s->max_depth4 - 6, 2), 9) / 3;
   return path_lanes(s->ctx) * (8 + std::min(s->max_depth4, 16)) / 4;
 }
 
