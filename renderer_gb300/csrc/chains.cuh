@@ -500,7 +500,7 @@ static unsigned long long run_wave(gbrt_scene* s, const Wave& w, const PTParams&
   unsigned long long launches = 3ull * unsigned(P.D);
   for (int it = 0; it < P.D; ++it) {
     const int cur = it & 1;
-    if (w.pk.finish && it >= kFinishFrom) {
+    if (w.pk.finish && finish_before(s, it, P.D)) {
       launch_finish(w.pk, s, P, st, cur, stream);
       ++launches;
     }

@@ -1656,7 +1656,22 @@ static void launch_finish(const PathKernels& pk, const gbrt_scene* s, const PTPa
   const int limit = int(std::min<long long>(path_lanes(s->ctx), P.nb));
   pk.finish<<<(limit + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, stream>>>(s->view, P, st, cur, limit);
 }
-constexpr int kFinishFrom = 2;  // first bounce that k_finish is launched before
+// Whether k_finish is launched before bounce `it`: before 2, 3, 4, 6, 8, 12, 16
+// and so on, since a launch that finds too many rays, or none, still costs a few
+// microseconds (Cornell box, 262k paths of up to 64 bounces, terminated with
+// probability 0.05: never / before every bounce / so 1924 / 2003 / 1673 us), and
+// only while enough bounces are left for their launches to cost more than
+// the longest path's latency. That is four in a shallow tree (five bounces,
+// never / before every one: CSG objects 285 / 339 us, Cornell box by the
+// physical estimator 254 / 262 with 262k paths) and any number in a deep one,
+// where each launch takes as long as its longest ray (icosphere of 327,680
+// triangles, 384k paths of five bounces 1090 / 869). With instances from 12
+// levels on (four meshes in a room, nine levels, 102k paths 606 / 701).
+static bool finish_before(const gbrt_scene* s, int it, int D) {
+  const bool deep = s->max_depth4 >= (s->view.inst ? 12 : 8);
+  auto pow2 = [](int x) { return (x & (x - 1)) == 0; };
+  return it >= 2 && D - it >= (deep ? 1 : 4) && (pow2(it) || (it % 3 == 0 && pow2(it / 3)));
+}
 
 static void init_params(PTParams& P, const gbrt_ctx* ctx, const gbrt_camera& cam, const gbrt_render_params& prm,
                         unsigned long long total) {
@@ -1801,7 +1816,7 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
       ++launches;
       for (int it = 0; it < P.D; ++it) {
         int cur = it & 1;
-        if (pk.finish && it >= kFinishFrom) {
+        if (pk.finish && finish_before(s, it, P.D)) {
           launch_finish(pk, s, P, st, cur, stream);
           ++launches;
         }
@@ -2340,7 +2355,7 @@ static gbrt_status render_guided_impl(gbrt_scene* s, const gbrt_camera* cam, con
         k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
         for (int it = 0; it < P.D; ++it) {
           int cur = it & 1;
-          if (pk.finish && it >= kFinishFrom) launch_finish(pk, s, P, st, cur, stream);
+          if (pk.finish && finish_before(s, it, P.D)) launch_finish(pk, s, P, st, cur, stream);
           tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
           if (P.guided && (P.guide_depth == 0 || it < P.guide_depth)) {
             cudaEvent_t ea = nullptr, eb = nullptr;
