@@ -725,8 +725,8 @@ __global__ void __launch_bounds__(256) k_pack_mixtures(const float4* __restrict_
 }
 
 constexpr int kMixFloats = 40;
-// Rows of gbrt_guide_eval in flight: bounds its workspace to 450 MB; a million
-// rows fill the GPU many times.
+// Rows of gbrt_guide_eval in flight: bounds its workspace to 420 MB and the
+// inputs; a million rows fill the GPU many times.
 constexpr size_t kEvalRows = size_t(1) << 20;
 
 }  // namespace
@@ -853,15 +853,15 @@ gbrt_status gbrt_guide_eval(gbrt_guide* g, const float* inputs, size_t n, float*
   const size_t rows = std::min(n, kEvalRows);
   float *d_raw = nullptr, *d_res = nullptr;
   float4 *d_in = nullptr, *d_mix = nullptr;
-  cudaError_t e = ctx_alloc(g->ctx, &d_raw, rows * 9 * sizeof(float), s);
+  cudaError_t e = ctx_alloc(g->ctx, &d_raw, n * 9 * sizeof(float), s);
   if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_in, rows * 3 * sizeof(float4), s);
   if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_mix, rows * kMixStride * sizeof(float4), s);
   if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_res, rows * kMixFloats * sizeof(float), s);
+  // All inputs first: out may be the same memory.
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_raw, inputs, n * 9 * sizeof(float), cudaMemcpyHostToDevice, s);
   for (size_t i = 0; i < n && e == cudaSuccess; i += rows) {
     const size_t m = std::min(rows, n - i);
-    e = cudaMemcpyAsync(d_raw, inputs + 9 * i, m * 9 * sizeof(float), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) break;
-    k_pack_rows<9, 3><<<unsigned((3 * m + 255) / 256), 256, 0, s>>>(d_raw, unsigned(m), d_in);
+    k_pack_rows<9, 3><<<unsigned((3 * m + 255) / 256), 256, 0, s>>>(d_raw + 9 * i, unsigned(m), d_in);
     e = launch_infer(g, d_in, nullptr, int(m), d_mix, s);
     if (e != cudaSuccess) break;
     k_pack_mixtures<<<unsigned((10 * m + 255) / 256), 256, 0, s>>>(d_mix, unsigned(m),
