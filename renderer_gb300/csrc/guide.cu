@@ -728,6 +728,11 @@ constexpr int kMixFloats = 40;
 // Rows of gbrt_guide_eval in flight: bounds its workspace to 420 MB and the
 // inputs; a million rows fill the GPU many times.
 constexpr size_t kEvalRows = size_t(1) << 20;
+// Evaluations of up to this many rows are laid out on the host: there the call's
+// time is its launches and copies, and the two kernels cost more than the loop
+// (laid out on the device / on the host: 1 row 46 / 41 us, 500 rows 58 / 50,
+// 1000 rows 60 / 63, 2000 rows 68 / 75).
+constexpr size_t kHostRows = 512;
 
 }  // namespace
 
@@ -851,29 +856,40 @@ gbrt_status gbrt_guide_eval(gbrt_guide* g, const float* inputs, size_t n, float*
   if (n > (1u << 26)) return fail(g->ctx, GBRT_ERR_INVALID_ARG, "gbrt_guide_eval: too many rows");
   cudaStream_t s = g->ctx->stream;
   const size_t rows = std::min(n, kEvalRows);
-  float *d_raw = nullptr, *d_res = nullptr;
-  float4 *d_in = nullptr, *d_mix = nullptr;
-  cudaError_t e = ctx_alloc(g->ctx, &d_raw, n * 9 * sizeof(float), s);
-  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_in, rows * 3 * sizeof(float4), s);
-  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_mix, rows * kMixStride * sizeof(float4), s);
-  if (e == cudaSuccess) e = ctx_alloc(g->ctx, &d_res, rows * kMixFloats * sizeof(float), s);
-  // All inputs first: out may be the same memory.
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_raw, inputs, n * 9 * sizeof(float), cudaMemcpyHostToDevice, s);
-  for (size_t i = 0; i < n && e == cudaSuccess; i += rows) {
-    const size_t m = std::min(rows, n - i);
-    k_pack_rows<9, 3><<<unsigned((3 * m + 255) / 256), 256, 0, s>>>(d_raw + 9 * i, unsigned(m), d_in);
-    e = launch_infer(g, d_in, nullptr, int(m), d_mix, s);
-    if (e != cudaSuccess) break;
-    k_pack_mixtures<<<unsigned((10 * m + 255) / 256), 256, 0, s>>>(d_mix, unsigned(m),
-                                                                    reinterpret_cast<float4*>(d_res));
-    e = cudaGetLastError();
+  const size_t inBytes = rows * 3 * sizeof(float4), mixBytes = rows * kMixStride * sizeof(float4);
+  const bool onHost = n <= kHostRows;
+  // One allocation, in parts of multiples of 16 bytes.
+  unsigned char* work = nullptr;
+  cudaError_t e = ctx_alloc(
+      g->ctx, &work, inBytes + mixBytes + (onHost ? 0 : (rows * kMixFloats + n * 9) * sizeof(float)), s);
+  float4* d_in = reinterpret_cast<float4*>(work);
+  float4* d_mix = reinterpret_cast<float4*>(work + inBytes);
+  float4 h[3 * kHostRows];  // the copy's source until the stream is waited for
+  if (onHost) {
+    for (size_t j = 0; j < 3 * n; ++j) h[j] = make_float4(inputs[3 * j], inputs[3 * j + 1], inputs[3 * j + 2], 0.f);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, h, inBytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = launch_infer(g, d_in, nullptr, int(n), d_mix, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(out + kMixFloats * i, d_res, m * kMixFloats * sizeof(float), cudaMemcpyDeviceToHost, s);
+      e = cudaMemcpy2DAsync(out, kMixFloats * sizeof(float), d_mix, kMixStride * sizeof(float4),
+                            kMixFloats * sizeof(float), n, cudaMemcpyDeviceToHost, s);
+  } else {
+    float* d_res = reinterpret_cast<float*>(work + inBytes + mixBytes);
+    float* d_raw = d_res + rows * kMixFloats;
+    // All inputs first: out may be the same memory.
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_raw, inputs, n * 9 * sizeof(float), cudaMemcpyHostToDevice, s);
+    for (size_t i = 0; i < n && e == cudaSuccess; i += rows) {
+      const size_t m = std::min(rows, n - i);
+      k_pack_rows<9, 3><<<unsigned((3 * m + 255) / 256), 256, 0, s>>>(d_raw + 9 * i, unsigned(m), d_in);
+      e = launch_infer(g, d_in, nullptr, int(m), d_mix, s);
+      if (e != cudaSuccess) break;
+      k_pack_mixtures<<<unsigned((10 * m + 255) / 256), 256, 0, s>>>(d_mix, unsigned(m),
+                                                                      reinterpret_cast<float4*>(d_res));
+      e = cudaGetLastError();
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(out + kMixFloats * i, d_res, m * kMixFloats * sizeof(float), cudaMemcpyDeviceToHost, s);
+    }
   }
-  if (d_raw) cudaFreeAsync(d_raw, s);
-  if (d_in) cudaFreeAsync(d_in, s);
-  if (d_mix) cudaFreeAsync(d_mix, s);
-  if (d_res) cudaFreeAsync(d_res, s);
+  if (work) cudaFreeAsync(work, s);
   const cudaError_t f = cudaStreamSynchronize(s);  // after an error too: the copies use the caller's memory
   if (e == cudaSuccess) e = f;
   if (e != cudaSuccess) return cuda_fail(g->ctx, e, "gbrt_guide_eval");
