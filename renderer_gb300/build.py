@@ -26,8 +26,9 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 # The path tracer's arithmetic has its fused multiply-adds spelled out: a path
 # comes out the same bit for bit in every kernel that runs it (one bounce per
 # launch, whole paths, many images). Left to the compiler, which product of a
-# sum is fused depends on the code around it.
-FLAGS = {"pathtrace.cu": ["-fmad=false"]}
+# sum is fused depends on the code around it. The macro says so to the source,
+# which does not compile without it.
+FLAGS = {"pathtrace.cu": ["-fmad=false", "-DGBRT_FMA_SPELLED_OUT"]}
 
 
 def nvcc():

@@ -24,6 +24,9 @@
 //               shadow  (any hit; unoccluded contributions added to the path)
 //   accumulate  per-pixel FP64 sum and sum of squares
 // Queue sizes live in device memory, so launch grids never depend on them.
+#ifndef GBRT_FMA_SPELLED_OUT
+#error "compile with -fmad=false -DGBRT_FMA_SPELLED_OUT (build.py FLAGS): contracted, the kernels stop agreeing bit for bit"
+#endif
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
