@@ -284,12 +284,16 @@ typedef struct gbrt_render_params {
 
 typedef enum gbrt_render_flags {
   /* Time every extend / shade / shadow kernel with CUDA events on the
-   * render stream (gbrt_stats *_ms fields). Either flag makes the render
-   * launch these kernels for every bounce; without them small wavefronts and
-   * the last paths of large ones run whole in one launch. */
+   * render stream (gbrt_stats *_ms fields). With either flag gbrt_render,
+   * gbrt_render_device and gbrt_render_passes launch these kernels for every
+   * bounce; without them small wavefronts and the last paths of large ones
+   * run whole in one launch, as they may in every other call:
+   * gbrt_render_guided times its inference and training with this flag
+   * (gbrt_guide_stats), gbrt_render_device_noalloc ignores it. */
   GBRT_RENDER_TIME_KERNELS = 1,
   /* Count BVH nodes visited and primitives tested (gbrt_stats counters);
-   * slower, for measurement only. */
+   * slower, for measurement only. gbrt_render_device_noalloc counts too, by
+   * the kernels per bounce; the guided, chain and batch renders do not. */
   GBRT_RENDER_COUNT_TRAVERSAL = 2
 } gbrt_render_flags;
 
