@@ -364,13 +364,20 @@ gbrt_status gbrt_ctx_trim(gbrt_ctx* ctx, uint64_t* reserved_bytes);
  *                          tensor-core products and give up waiting for them
  *                          after arg ns (the call returns GBRT_ERR_TIMEOUT,
  *                          the kernels' tensor memory is freed); 0 turns it off.
+ *   GBRT_FAULT_LATE_LAUNCHES  arg != 0: wavefronts are not run whole, the
+ *                          kernel that ends their last paths gets all of them
+ *                          before the third bounce, and the launches of that
+ *                          bounce and of the later ones are left out: an image
+ *                          is whole only if that kernel ran every path. (Not
+ *                          for scenes and flags that keep the kernels per bounce.)
  */
 typedef enum gbrt_fault {
   GBRT_FAULT_NONE = 0,
   GBRT_FAULT_ALLOC = 1,
   GBRT_FAULT_NAN = 2,
   GBRT_FAULT_SMALL_STACK = 3,
-  GBRT_FAULT_GUIDE_WAIT = 4
+  GBRT_FAULT_GUIDE_WAIT = 4,
+  GBRT_FAULT_LATE_LAUNCHES = 5
 } gbrt_fault;
 gbrt_status gbrt_debug_fault(gbrt_ctx* ctx, int32_t kind, int64_t arg);
 

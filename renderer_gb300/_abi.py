@@ -168,7 +168,7 @@ SCENE_WATERTIGHT, SCENE_GPU_BUILD, SCENE_ENV_UNIFORM, SCENE_LIST_ORDER = 1, 2, 4
 RENDER_TIME_KERNELS, RENDER_COUNT_TRAVERSAL = 1, 2
 NOALLOC_MAX_BATCH = 65536
 # gbrt_fault (host-side fault injection for the failure-path tests)
-FAULT_NONE, FAULT_ALLOC, FAULT_NAN, FAULT_SMALL_STACK, FAULT_GUIDE_WAIT = 0, 1, 2, 3, 4
+FAULT_NONE, FAULT_ALLOC, FAULT_NAN, FAULT_SMALL_STACK, FAULT_GUIDE_WAIT, FAULT_LATE_LAUNCHES = range(6)
 GUIDE_PARAMS, GUIDE_INPUT, GUIDE_OUTPUT, GUIDE_SAMPLE = 24064, 9, 40, 13
 CSG_SPHERE, CSG_BOX, CSG_ISECT, CSG_UNION, CSG_DIFF, CSG_XOR = range(6)
 CSG_MAX_LEAVES = 8

@@ -497,12 +497,13 @@ static unsigned long long run_wave(gbrt_scene* s, const Wave& w, const PTParams&
     w.pk.finish<<<(P.nb + block - 1) / block, block, 0, stream>>>(s->view, P, st, 0, P.nb);
     return 1;
   }
-  unsigned long long launches = 3ull * unsigned(P.D);
+  unsigned long long launches = 0;
   for (int it = 0; it < P.D; ++it) {
     const int cur = it & 1;
     if (w.pk.finish && finish_before(s, it, P.D)) {
       launch_finish(w.pk, s, P, st, cur, stream);
       ++launches;
+      if (s->ctx->fault_late_launches) break;
     }
     // The first rays too: the chains' points lie all over the image, so these
     // rays are as different as later ones (icosphere of 81,920 triangles, a
@@ -511,6 +512,7 @@ static unsigned long long run_wave(gbrt_scene* s, const Wave& w, const PTParams&
     w.tk.ext<<<cap_grid(w.traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
     w.shade<<<cap_grid(w.shadeGrid, P.nb, 256), 256, 0, stream>>>(s->view, P, st, cur);
     w.tk.sh<<<cap_grid(w.shadowGrid, 2ll * P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st);
+    launches += 3;
   }
   return launches;
 }

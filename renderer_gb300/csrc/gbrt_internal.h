@@ -38,6 +38,7 @@ struct gbrt_ctx {
   mutable long long fault_alloc_countdown = -1;  // device allocations that still succeed (-1: off)
   unsigned long long fault_nan_every = 0;        // every n-th camera sample's radiance becomes NaN
   bool fault_small_stack = false;                // traversal kernels with a kFaultStack-entry stack
+  bool fault_late_launches = false;              // no launches of bounces after k_finish's, which takes all paths
   unsigned long long fault_guide_wait_ns = 0;    // guide kernels skip their products and wait this long
 };
 

@@ -1638,6 +1638,7 @@ static long long path_lanes(const gbrt_ctx* ctx) { return 512ll * ctx->num_sms; 
 // 2216 / 2142 at 262k; an open terrain (15 levels, three bounces) 645 / 637 at
 // 262k. So 2/3 of a path per lane up to eight levels, 1/3 more a level, at most 3.
 static long long whole_path_limit(const gbrt_scene* s) {
+  if (s->ctx->fault_late_launches) return 0;
   if (s->view.inst) return path_lanes(s->ctx) * std::min(std::max(s->max_depth4 - 6, 2), 9) / 3;
   return path_lanes(s->ctx) * (8 + std::min(s->max_depth4, 16)) / 4;
 }
@@ -1656,7 +1657,7 @@ static void launch_path(const PathKernels& pk, const gbrt_scene* s, const PTPara
 // rooms and the Cornell box).
 static void launch_finish(const PathKernels& pk, const gbrt_scene* s, const PTParams& P, const PTState& st, int cur,
                           cudaStream_t stream) {
-  const int limit = int(std::min<long long>(path_lanes(s->ctx), P.nb));
+  const int limit = s->ctx->fault_late_launches ? P.nb : int(std::min<long long>(path_lanes(s->ctx), P.nb));
   pk.finish<<<(limit + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, stream>>>(s->view, P, st, cur, limit);
 }
 // Whether k_finish is launched before bounce `it`: before 2, 3, 4, 6, 8, 12, 16
@@ -1671,6 +1672,7 @@ static void launch_finish(const PathKernels& pk, const gbrt_scene* s, const PTPa
 // triangles, 384k paths of five bounces 1090 / 869). With instances from 12
 // levels on (four meshes in a room, nine levels, 102k paths 606 / 701).
 static bool finish_before(const gbrt_scene* s, int it, int D) {
+  if (s->ctx->fault_late_launches) return it == 2;
   const bool deep = s->max_depth4 >= (s->view.inst ? 12 : 8);
   auto pow2 = [](int x) { return (x & (x - 1)) == 0; };
   return it >= 2 && D - it >= (deep ? 1 : 4) && (pow2(it) || (it % 3 == 0 && pow2(it / 3)));
@@ -1822,6 +1824,7 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
         if (pk.finish && finish_before(s, it, P.D)) {
           launch_finish(pk, s, P, st, cur, stream);
           ++launches;
+          if (ctx->fault_late_launches) break;
         }
         if (timeK) mark();
         tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
@@ -2358,7 +2361,10 @@ static gbrt_status render_guided_impl(gbrt_scene* s, const gbrt_camera* cam, con
         k_raygen<<<(P.nb + 255) / 256, 256, 0, stream>>>(P, st);
         for (int it = 0; it < P.D; ++it) {
           int cur = it & 1;
-          if (pk.finish && finish_before(s, it, P.D)) launch_finish(pk, s, P, st, cur, stream);
+          if (pk.finish && finish_before(s, it, P.D)) {
+            launch_finish(pk, s, P, st, cur, stream);
+            if (ctx->fault_late_launches) break;
+          }
           tk.extend(it)<<<cap_grid(traceGrid, P.nb, kTraceBlock), kTraceBlock, 0, stream>>>(s->view, st, cur);
           if (P.guided && (P.guide_depth == 0 || it < P.guide_depth)) {
             cudaEvent_t ea = nullptr, eb = nullptr;

@@ -343,6 +343,7 @@ gbrt_status gbrt_debug_fault(gbrt_ctx* ctx, int32_t kind, int64_t arg) {
       ctx->fault_nan_every = 0;
       ctx->fault_small_stack = false;
       ctx->fault_guide_wait_ns = 0;
+      ctx->fault_late_launches = false;
       return GBRT_OK;
     case GBRT_FAULT_ALLOC:
       if (arg < 0) return fail(ctx, GBRT_ERR_INVALID_ARG, "gbrt_debug_fault: negative allocation count");
@@ -354,6 +355,9 @@ gbrt_status gbrt_debug_fault(gbrt_ctx* ctx, int32_t kind, int64_t arg) {
       return GBRT_OK;
     case GBRT_FAULT_SMALL_STACK:
       ctx->fault_small_stack = arg != 0;
+      return GBRT_OK;
+    case GBRT_FAULT_LATE_LAUNCHES:
+      ctx->fault_late_launches = arg != 0;
       return GBRT_OK;
     case GBRT_FAULT_GUIDE_WAIT:
       if (arg < 0 || arg > 1000000000) return fail(ctx, GBRT_ERR_INVALID_ARG, "gbrt_debug_fault: wait outside [0, 1 s]");
