@@ -24,6 +24,8 @@
 //               shadow  (any hit; unoccluded contributions added to the path)
 //   accumulate  per-pixel FP64 sum and sum of squares
 // Queue sizes live in device memory, so launch grids never depend on them.
+// Small wavefronts run whole paths in one launch instead (k_path), and the last
+// paths of large ones end in one (k_finish, launched before some bounces).
 #ifndef GBRT_FMA_SPELLED_OUT
 #error "compile with -fmad=false -DGBRT_FMA_SPELLED_OUT (build.py FLAGS): contracted, the kernels stop agreeing bit for bit"
 #endif
@@ -639,7 +641,7 @@ __device__ __forceinline__ void nee(const DeviceScene& S, const PTParams& P, ST&
 // estimation in each branch a warp ran up to four of them one after the other.
 // Cornell box, 2^20 paths: 1.19 -> 1.06 ms a frame; ten small mesh scenes in
 // shared wavefronts 12.4 -> 11.0 ms; the 67M-path icosphere frame 51.5 ->
-// 49.8 ms (latency and the path state's traffic bound it there).
+// 49.8 ms (there instruction fetch bound it, see out_direction).
 template <bool EXT, class R, class ST>
 __device__ __forceinline__ void shade_vertex(const DeviceScene& S, const PTParams& P, ST& ss, const R& rs,
                                              const RawHit& h, const int* hit_inst, float4 ro, float4 rd, int* err) {
@@ -1625,10 +1627,13 @@ static long long path_lanes(const gbrt_ctx* ctx) { return 512ll * ctx->num_sms; 
 // Wavefronts of up to this many paths take k_path. What it saves, the
 // latency of 3 D nearly empty launches, grows with the tree's depth; what it
 // costs, lanes that idle while their warp's longest path goes on, grows with
-// the paths per lane. Measured (frame time by bounces / by k_path, us): Cornell
-// box (one level) 131k paths 425 / 342, 262k 540 / 588; two rooms of 500,000
-// triangles 262k 1330 / 888, 524k 1729 / 1623; icosphere of 1.31M 262k
-// 2036 / 816, 1M 3132 / 2454.
+// the paths per lane. Measured (time of a call by bounces / by k_path, us, eight
+// bounces): Cornell box (one level) 131k paths 382 / 236, 262k 498 / 479, 393k
+// 527 / 575; textured box (two levels) 131k 415 / 286, 197k 473 / 486; two rooms of
+// 500,000 triangles (ten levels) 262k 865 / 686, 524k 1263 / 1297; icosphere of
+// 1.31M (twelve levels) 262k 1217 / 688, 524k 1277 / 852, 1M 1981 / 2021. The
+// limit stays below these crossings (175k, 195k, 350k and 389k paths on 152 SMs),
+// near them only in the textured box.
 // With instances the costs are higher (the ray in two spaces, the CSG code: fewer
 // lanes at work in a bigger kernel) and the line lies lower. Five bounces, by
 // bounces / by k_path, us, at 1 / 2 / 3 paths per lane and above: four meshes in
@@ -1753,7 +1758,10 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
   // Per-kernel times and counters want the kernels per bounce.
   const PathKernels pk = timeK || count ? PathKernels{} : pick_path(s, P.physical != 0);
   // Every wavefront by k_path: of a path only its radiance is stored (the
-  // preview of 3,015 paths: 24 allocations cost 30 us of its 139).
+  // preview of 3,015 paths: 24 allocations cost 30 us of its 139). alpha, ctl,
+  // counts and work are not read then; these four smallest allocations (5 us)
+  // only keep a call's allocations at the eight that the injected failure of one
+  // in the middle (GBRT_FAULT_ALLOC, n = 7) is tested on.
   const bool whole = pk.path && B <= whole_path_limit(s);
   A(buf.alloc(&st.L, B));
   A(buf.alloc(&st.alpha, whole ? 1 : B)); A(buf.alloc(&st.ctl, whole ? 1 : B));
