@@ -1758,15 +1758,16 @@ static gbrt_status render_impl(gbrt_scene* s, const gbrt_camera* cam, const gbrt
   // Per-kernel times and counters want the kernels per bounce.
   const PathKernels pk = timeK || count ? PathKernels{} : pick_path(s, P.physical != 0);
   // Every wavefront by k_path: of a path only its radiance is stored (the
-  // preview of 3,015 paths: 24 allocations cost 30 us of its 139). alpha, ctl,
-  // counts and work are not read then; these four smallest allocations (5 us)
-  // only keep a call's allocations at the eight that the injected failure of one
-  // in the middle (GBRT_FAULT_ALLOC, n = 7) is tested on.
+  // preview of 3,015 paths: 24 allocations cost 30 us of its 139). The four arrays
+  // left out first count for an injected failure all the same, so that the n-th
+  // allocation is the same one as before them.
   const bool whole = pk.path && B <= whole_path_limit(s);
   A(buf.alloc(&st.L, B));
-  A(buf.alloc(&st.alpha, whole ? 1 : B)); A(buf.alloc(&st.ctl, whole ? 1 : B));
-  A(buf.alloc(&st.counts, 4)); A(buf.alloc(&st.work, 4));
-  if (!whole) {
+  if (whole) {
+    for (int k = 0; k < 4; ++k) A(fault_alloc(ctx));
+  } else {
+    A(buf.alloc(&st.alpha, B)); A(buf.alloc(&st.ctl, B));
+    A(buf.alloc(&st.counts, 4)); A(buf.alloc(&st.work, 4));
     A(buf.alloc(&st.pv_p, B)); A(buf.alloc(&st.pv_n, B)); A(buf.alloc(&st.pv_d, B)); A(buf.alloc(&st.pv_a, B));
     A(buf.alloc(&st.ext[0], 2 * B)); A(buf.alloc(&st.ext[1], 2 * B));
     A(buf.alloc(&st.ext_slot[0], B)); A(buf.alloc(&st.ext_slot[1], B));
